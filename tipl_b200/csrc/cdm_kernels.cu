@@ -118,10 +118,20 @@ __device__ void control_block(const CdmSeg& S, int mod);
 __device__ __forceinline__ bool last_block_of_segment(const CdmSeg& S);
 
 // ------------------------------------------------------------------ gradient
-// Window sums of linear_regression over the clipped 5^3 window
-// (numerical/window.hpp:92-110, numerical/statistics.hpp:694-713).  Integer
-// pixels: exact integer sums (the reference sums in int64).  Float pixels: double
-// sums in the reference's visiting order with float cross products.
+// x / m rounded like the division, for the window sizes m <= 125 and r = RN(1 / m): the
+// quotient from the reciprocal, corrected twice by its exact remainder.  With r correctly
+// rounded and the first correction within an ulp, the second rounds correctly (Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000 processor", 1990).  An
+// infinite x makes the remainder NaN; the division itself settles those.
+__device__ __forceinline__ double div_window(double x, double m, double r)
+{
+    double q = x * r;
+    q = __fma_rn(__fma_rn(-q, m, x), r, q);
+    q = __fma_rn(__fma_rn(-q, m, x), r, q);
+    return q == q ? q : x / m;
+}
+
+// The regression of the clipped 5^3 window's sums (numerical/statistics.hpp:694-713).
 struct Reg {
     float a, b, r2;
 };
@@ -129,68 +139,21 @@ struct Reg {
 __device__ __forceinline__ void regress_finish(double sx, double sy, double sxx, double syy, double sxy, int m,
                                                Reg& r)
 {
-    const double dn = (double)m;
-    const double mx = sx / dn, my = sy / dn;
-    const double xv = sxx / dn - mx * mx;
-    const double yv = syy / dn - my * my;
+    const double dn = (double)m, rn = 1.0 / dn;
+    const double mx = div_window(sx, dn, rn), my = div_window(sy, dn, rn);
+    const double xv = div_window(sxx, dn, rn) - mx * mx;
+    const double yv = div_window(syy, dn, rn) - my * my;
     if (xv == 0.0 || yv == 0.0) {
         r.a = 0.0f;
         r.b = (float)my;
         r.r2 = 0.0f;
         return;
     }
-    const double cov = sxy / dn - mx * my;
+    const double cov = div_window(sxy, dn, rn) - mx * my;
     r.a = (float)(cov / xv);
     r.b = (float)(my - (double)r.a * mx);  // b uses the float-rounded slope
     r.r2 = (float)(cov * cov / xv / yv);
 }
-
-template <typename T>
-struct WindowAcc;
-
-template <>
-struct WindowAcc<uint8_t> {
-    int sx = 0, sy = 0, sxx = 0, syy = 0, sxy = 0, m = 0;
-    __device__ __forceinline__ void add(uint8_t j, uint8_t t)
-    {
-        const int a = j, b = t;
-        sx += a;
-        sy += b;
-        sxx += a * a;
-        syy += b * b;
-        sxy += a * b;
-        ++m;
-    }
-    __device__ __forceinline__ void finish(Reg& r) const
-    {
-        regress_finish((double)sx, (double)sy, (double)sxx, (double)syy, (double)sxy, m, r);
-    }
-};
-
-template <>
-struct WindowAcc<float> {
-    double sx = 0, sy = 0, sxx = 0, syy = 0, sxy = 0;
-    int m = 0;
-    __device__ __forceinline__ void add(float j, float t)
-    {
-        // sum(): first element then +=; square_sum(): 0 + t*t in double;
-        // inner_product(): float product widened to double.
-        if (m == 0) {
-            sx = (double)j;
-            sy = (double)t;
-            sxy = (double)(j * t);
-        } else {
-            sx += (double)j;
-            sy += (double)t;
-            sxy += (double)(j * t);
-        }
-        const double dj = j, dt = t;
-        sxx += dj * dj;
-        syy += dt * dt;
-        ++m;
-    }
-    __device__ __forceinline__ void finish(Reg& r) const { regress_finish(sx, sy, sxx, syy, sxy, m, r); }
-};
 
 template <typename T>
 __device__ __forceinline__ float pix_diff(T a, T b)
@@ -229,12 +192,10 @@ __device__ __forceinline__ void store_term(float* __restrict__ nd, long long i, 
     nd[3 * i + 2] = out.z;
 }
 
-// cdm_get_gradient_r_imp / _d_imp (reg/cdm.hpp:46-78) of modality mod: the term is
-// 0 + gradient term; the cost of every voxel (0 where skipped) is summed per block in
-// double.
+// cdm_get_gradient_d_imp (reg/cdm.hpp:46-78) of modality mod: the term is 0 + gradient
+// term; the cost of every voxel is summed per block in double.
 template <typename T, bool MULTI>
-__global__ void __launch_bounds__(kCdmThreads) cdm_gradient_kernel(const CdmSeg* __restrict__ segs, int nseg, int gtype,
-                                                                   int mod)
+__global__ void __launch_bounds__(kCdmThreads) cdm_gradient_d_kernel(const CdmSeg* __restrict__ segs, int nseg, int mod)
 {
     SEG_BEGIN
     if (S.ctl->done || mod >= max(S.nmod, 1))
@@ -246,77 +207,13 @@ __global__ void __launch_bounds__(kCdmThreads) cdm_gradient_kernel(const CdmSeg*
     for (long long i = first; i < n; i += stride) {
         int x, y, z;
         unflat((int)i, D, x, y, z);
-        float3 out = make_float3(0.0f, 0.0f, 0.0f);
-        float cost = 0.0f;
-        const T js = Js[i], it = It[i];
-        if (gtype == 'd') {
-            float3 g = grad_at(Js, D, x, y, z, i);
-            const float dif = pix_diff(js, it);
-            g.x *= dif;
-            g.y *= dif;
-            g.z *= dif;
-            out.x = 0.0f + g.x;
-            out.y = 0.0f + g.y;
-            out.z = 0.0f + g.z;
-            cost = dif * dif;
-        } else if (!(js == T(0) || it == T(0))) {
-            const int xu = min(D.w - x - 1, 2), yu = min(D.h - y - 1, 2), zu = min(D.d - z - 1, 2);
-            const int xl = min(x, 2), yl = min(y, 2), zl = min(z, 2);
-            const long long w = D.w, wh = D.wh();
-            WindowAcc<T> acc;
-            // (float pixels only: the uint8 'r' gradient is the box-sum kernel below)
-            if (sizeof(T) == 4 && xu == 2 && xl == 2 && yu == 2 && yl == 2 && zu == 2 && zl == 2) {
-                // an interior voxel: the whole 5^3 window, visited in the same order
-                // with every offset known -- no loop bounds, no index arithmetic per tap
-                const T* __restrict__ pj = Js + i;
-                const T* __restrict__ pt = It + i;
-                constexpr int kOrd[5] = {0, 1, 2, -1, -2};
-#pragma unroll
-                for (int a = 0; a < 5; ++a) {
-#pragma unroll
-                    for (int b = 0; b < 5; ++b) {
-                        const long long row = kOrd[a] * wh + kOrd[b] * w;
-                        const T* __restrict__ rj = pj + row;
-                        const T* __restrict__ rt = pt + row;
-#pragma unroll
-                        for (int c = 0; c < 5; ++c)
-                            acc.add(rj[kOrd[c]], rt[kOrd[c]]);
-                    }
-                }
-            } else
-            // iterate_xyz order (numerical/window.hpp:54-72)
-            for (int pz = 0; pz < 2; ++pz) {
-                const int zc = pz ? zl : zu;
-                for (int dz = pz; dz <= zc; ++dz) {
-                    const long long zi = i + (pz ? -dz : dz) * wh;
-                    for (int py = 0; py < 2; ++py) {
-                        const int yc = py ? yl : yu;
-                        for (int dy = py; dy <= yc; ++dy) {
-                            const long long yi = zi + (py ? -dy : dy) * w;
-                            for (int dx = 0; dx <= xu; ++dx)
-                                acc.add(Js[yi + dx], It[yi + dx]);
-                            for (int dx = 1; dx <= xl; ++dx)
-                                acc.add(Js[yi - dx], It[yi - dx]);
-                        }
-                    }
-                }
-            }
-            Reg r;
-            acc.finish(r);
-            if (r.a > 0.0f) {
-                float3 g = grad_at(Js, D, x, y, z, i);
-                const float s = r.r2 * ((float)js * r.a + r.b - (float)it);
-                g.x *= s;
-                g.y *= s;
-                g.z *= s;
-                out.x = 0.0f + g.x;
-                out.y = 0.0f + g.y;
-                out.z = 0.0f + g.z;
-                cost = -r.r2;
-            }
-        }
-        store_term(nd, i, out, mod);
-        csum += (double)cost;
+        float3 g = grad_at(Js, D, x, y, z, i);
+        const float dif = pix_diff(Js[i], It[i]);
+        g.x *= dif;
+        g.y *= dif;
+        g.z *= dif;
+        store_term(nd, i, make_float3(0.0f + g.x, 0.0f + g.y, 0.0f + g.z), mod);
+        csum += (double)(dif * dif);
     }
     __shared__ double red[32];
     csum = block_sum(csum, red);
@@ -460,6 +357,188 @@ __global__ void __launch_bounds__(kBoxThreads) cdm_gradient_box_u8_kernel(const 
         control_block(S, mod);
 }
 
+// Asynchronous copy of a float from global to shared memory, +0 instead where !ok: all of a
+// tile's loads are in flight together.
+__device__ __forceinline__ void copy_async_f32(float* to, const float* from, bool ok)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((unsigned)__cvta_generic_to_shared(to)), "l"(from),
+                 "r"(ok ? 4 : 0)
+                 : "memory");
+}
+__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// Tiled float 'r' gradient (cdm_get_gradient_r_imp, reg/cdm.hpp:46-78).  Float pixels: the
+// window sums of linear_regression over the clipped 5^3 window (numerical/window.hpp:92-110,
+// numerical/statistics.hpp:694-713) are double sums in the reference's visiting order
+// (offsets 0, 1, 2, -1, -2 per axis, z outermost), sxy of float products.  Double sums do
+// not reassociate, so every voxel adds its own 125 taps in that order; taps outside the
+// volume are zeros of the staged tile, which change no sum.  What neighbouring voxels share
+// is the taps' widening to double and their products, so a thread takes V voxels in x:
+// with V = 4 a window row is 8 values, widened once (24 conversions) for 20 taps.  A square
+// of a widened float is exact, so adding it by a fused multiply-add rounds like the sum.
+// Bound by the conversion unit and the FP64 pipe (50 SM cycles each a window row of a warp of
+// 128 voxels); three blocks an SM and the tile's loads all in flight at once hide the rest.
+// 157x189x155 launch: 305 us with one voxel a thread reading global memory, 235 so;
+// 91x109x91: 87 / 66; 64^3: 50 / 32; 23x28x23: 25 / 14.6.
+constexpr int kFX = 32, kFY = 8, kFThreads = 256, kFHX = kFX + 4, kFHY = kFY + 4, kFMaxV = 4;
+
+template <int V>
+__device__ __forceinline__ double gradient_r_f32(const CdmSeg& S, int blk, int mod, float* __restrict__ smem)
+{
+    constexpr int kTX = kFX / V, kHZ = V + 4;  // the tile is 32 x 8 x V voxels
+    static_assert((V == 2 || V == 4) && kTX * kFY * V == kFThreads, "one thread per V voxels of the tile");
+    float* const sj = smem;
+    float* const si = smem + kHZ * kFHY * kFHX;
+    const Dim3 D{S.w, S.h, S.d};
+    const float* __restrict__ Js = (const float*)S.Js;
+    const float* __restrict__ It = (const float*)S.It[mod];
+    float* __restrict__ nd = S.new_d;
+    const int ntx = (D.w + kFX - 1) / kFX, nty = (D.h + kFY - 1) / kFY, ntz = (D.d + V - 1) / V;
+    const long long ntiles = (long long)ntx * nty * ntz;
+    const long long wl = D.w, whl = D.wh();
+    const int xo = V * (threadIdx.x % kTX), yo = threadIdx.x / kTX % kFY, zo = threadIdx.x / (kTX * kFY);
+    const int lane = threadIdx.x & 31;
+    double csum = 0.0;
+    for (long long tile = blk; tile < ntiles; tile += S.nblk) {
+        const int x0 = (int)(tile % ntx) * kFX, y0 = (int)(tile / ntx % nty) * kFY, z0 = (int)(tile / ((long long)ntx * nty)) * V;
+        __syncthreads();  // the previous tile's readers are done with the buffers
+        for (int r = threadIdx.x >> 5; r < kFHY * kHZ; r += kFThreads / 32) {
+            const int gy = y0 + r % kFHY - 2, gz = z0 + r / kFHY - 2;
+            const bool row = gy >= 0 && gz >= 0 && gy < D.h && gz < D.d;
+            const long long gi = gz * whl + gy * wl + x0 - 2;
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const int hx = lane + 32 * k, gx = x0 + hx - 2;
+                if (hx < kFHX) {
+                    const bool ok = row && gx >= 0 && gx < D.w;
+                    copy_async_f32(sj + r * kFHX + hx, ok ? Js + gi + hx : Js, ok);
+                    copy_async_f32(si + r * kFHX + hx, ok ? It + gi + hx : It, ok);
+                }
+            }
+        }
+        copy_async_wait();
+        __syncthreads();
+        const int y = y0 + yo, z = z0 + zo;
+        if (x0 + xo >= D.w || y >= D.h || z >= D.d)
+            continue;
+        const long long i0 = z * whl + y * wl + x0 + xo;
+        const float* const cj = sj + ((zo + 2) * kFHY + yo + 2) * kFHX + xo + 2;  // the first voxel in the tile
+        const float* const ci = si + (cj - sj);
+        bool any = false;
+#pragma unroll
+        for (int v = 0; v < V; ++v)
+            any = any || !(cj[v] == 0.0f || ci[v] == 0.0f);
+        double sx[V] = {}, sy[V] = {}, sxx[V] = {}, syy[V] = {}, sxy[V] = {};
+        if (any) {
+#pragma unroll 1
+            for (int row = 0; row < 25; ++row) {
+                const int a = row / 5, b = row % 5;  // offsets 0, 1, 2, -1, -2
+                const int o = ((zo + 2 + (a < 3 ? a : 2 - a)) * kFHY + yo + 2 + (b < 3 ? b : 2 - b)) * kFHX + xo;
+                float fj[V + 4], ft[V + 4];
+#pragma unroll
+                for (int k = 0; k < V + 4; k += V) {
+                    if constexpr (V == 4) {
+                        const float4 p = *reinterpret_cast<const float4*>(sj + o + k), q = *reinterpret_cast<const float4*>(si + o + k);
+                        fj[k] = p.x, fj[k + 1] = p.y, fj[k + 2] = p.z, fj[k + 3] = p.w;
+                        ft[k] = q.x, ft[k + 1] = q.y, ft[k + 2] = q.z, ft[k + 3] = q.w;
+                    } else {
+                        const float2 p = *reinterpret_cast<const float2*>(sj + o + k), q = *reinterpret_cast<const float2*>(si + o + k);
+                        fj[k] = p.x, fj[k + 1] = p.y;
+                        ft[k] = q.x, ft[k + 1] = q.y;
+                    }
+                }
+                // one quantity after the other: 8 widened values at a time
+                constexpr int kOrd[5] = {2, 3, 4, 1, 0};
+                double q[V + 4];
+#pragma unroll
+                for (int k = 0; k < V + 4; ++k)
+                    q[k] = (double)fj[k];
+#pragma unroll
+                for (int c = 0; c < 5; ++c)
+#pragma unroll
+                    for (int v = 0; v < V; ++v) {
+                        sx[v] += q[v + kOrd[c]];
+                        sxx[v] = __fma_rn(q[v + kOrd[c]], q[v + kOrd[c]], sxx[v]);
+                    }
+#pragma unroll
+                for (int k = 0; k < V + 4; ++k)
+                    q[k] = (double)ft[k];
+#pragma unroll
+                for (int c = 0; c < 5; ++c)
+#pragma unroll
+                    for (int v = 0; v < V; ++v) {
+                        sy[v] += q[v + kOrd[c]];
+                        syy[v] = __fma_rn(q[v + kOrd[c]], q[v + kOrd[c]], syy[v]);
+                    }
+#pragma unroll
+                for (int k = 0; k < V + 4; ++k)
+                    q[k] = (double)__fmul_rn(fj[k], ft[k]);
+#pragma unroll
+                for (int c = 0; c < 5; ++c)
+#pragma unroll
+                    for (int v = 0; v < V; ++v)
+                        sxy[v] += q[v + kOrd[c]];
+            }
+        }
+        const int myz = (min(D.h - 1, y + 2) - max(0, y - 2) + 1) * (min(D.d - 1, z + 2) - max(0, z - 2) + 1);
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+            const int x = x0 + xo + v;
+            if (x >= D.w)
+                break;
+            float3 out = make_float3(0.0f, 0.0f, 0.0f);
+            const float js = cj[v], it = ci[v];
+            if (!(js == 0.0f || it == 0.0f)) {
+                Reg r;
+                regress_finish(sx[v], sy[v], sxx[v], syy[v], sxy[v],
+                               (min(D.w - 1, x + 2) - max(0, x - 2) + 1) * myz, r);
+                if (r.a > 0.0f) {
+                    // gradient_at from the tile (neighbours are inside the halo)
+                    const float* const p = cj + v;
+                    float3 g;
+                    g.x = (x + 1 < D.w && x) ? p[1] - p[-1] : 0.0f;
+                    g.y = (y + 1 < D.h && y) ? p[kFHX] - p[-kFHX] : 0.0f;
+                    g.z = (z + 1 < D.d && z) ? p[kFHX * kFHY] - p[-kFHX * kFHY] : 0.0f;
+                    const float s = r.r2 * (js * r.a + r.b - it);
+                    g.x *= s;
+                    g.y *= s;
+                    g.z *= s;
+                    out.x = 0.0f + g.x;
+                    out.y = 0.0f + g.y;
+                    out.z = 0.0f + g.z;
+                    csum += (double)-r.r2;
+                }
+            }
+            store_term(nd, i0 + v, out, mod);
+        }
+    }
+    return csum;
+}
+
+template <bool MULTI>
+__global__ void __launch_bounds__(kFThreads, 3) cdm_gradient_r_f32_kernel(const CdmSeg* __restrict__ segs, int nseg,
+                                                                          int mod)
+{
+    const CdmSeg& S = segs[MULTI ? seg_of_block(segs, nseg) : 0];
+    const int blk = (int)blockIdx.x - (MULTI ? S.blk0 : 0);
+    if (blk >= S.nblk)
+        return;
+    if (S.ctl->done || mod >= max(S.nmod, 1))
+        return;
+    __shared__ __align__(16) float smem[2 * (kFMaxV + 4) * kFHY * kFHX];
+    // Small levels take two voxels a thread: a tile's time is its 25 rows' latency there, and
+    // there are not enough tiles of four to fill the chip (91x109x91: 71.0 us with two, 65.6
+    // with four; 64^3: 32.0 / 30.1; 46x55x46: 25.3 / 27.4; 23x28x23: 14.8 / 20.6).
+    const long long n = (long long)S.w * S.h * S.d;
+    const double cs = n < 200000 ? gradient_r_f32<2>(S, blk, mod, smem) : gradient_r_f32<4>(S, blk, mod, smem);
+    __shared__ double red[32];
+    const double csum = block_sum(cs, red);
+    if (threadIdx.x == 0)
+        S.cost_part[blk] = csum;
+    if (last_block_of_segment(S))
+        control_block(S, mod);
+}
+
 // ------------------------------------------------------------------ control
 // cdm_improved (reg/cdm.hpp:19-34): regression of the last costs on their index
 // (int x, float y; statistics.hpp:694-713); a positive slope means "not improved".
@@ -517,13 +596,8 @@ __device__ float seg_cost_mean(const CdmSeg& S)
 // gradient kernel's last block).  Each modality's launch keeps its mean cost; the
 // last modality's sums them in modality order (float), failing the level as soon
 // as a partial sum is exactly zero, and records sum / nmod.
-__device__ void control_block(const CdmSeg& S, int mod)
+__device__ void control_step(CdmCtl* c, int nm, int mod, float mean_cost)
 {
-    CdmCtl* c = S.ctl;
-    const float mean_cost = seg_cost_mean(S);
-    if (threadIdx.x != 0)
-        return;
-    const int nm = S.nmod > 1 ? S.nmod : 1;
     c->mod_cost[mod] = mean_cost;
     if (mod + 1 < nm)
         return;
@@ -562,6 +636,26 @@ __device__ void control_block(const CdmSeg& S, int mod)
     }
     ++c->index;
     ++c->iters_run;
+}
+
+// The block works on a copy of the control block in shared memory: one thread takes the
+// decisions, some thirty dependent loads and stores, each of which would cost a trip to L2
+// (16^3 uint8 gradient launch: 15.5 us with the control block in global memory, 14.7 so).
+__device__ void control_block(const CdmSeg& S, int mod)
+{
+    constexpr int kWords = sizeof(CdmCtl) / 4;
+    static_assert(sizeof(CdmCtl) % 4 == 0, "copied by words");
+    __shared__ CdmCtl c;
+    uint32_t* const g = reinterpret_cast<uint32_t*>(S.ctl);
+    uint32_t* const l = reinterpret_cast<uint32_t*>(&c);
+    for (int i = threadIdx.x; i < kWords; i += blockDim.x)
+        l[i] = g[i];
+    const float mean_cost = seg_cost_mean(S);  // (its barriers order the copy too)
+    if (threadIdx.x == 0)
+        control_step(&c, S.nmod > 1 ? S.nmod : 1, mod, mean_cost);
+    __syncthreads();
+    for (int i = threadIdx.x; i < kWords; i += blockDim.x)
+        g[i] = l[i];
 }
 
 // Completion ticket of a segment's blocks: true in the one block that finishes
@@ -1135,12 +1229,12 @@ cudaError_t launch_cdm_gradient(const CdmSeg* segs, int nseg, int blocks, int pi
         }
         SEG_LAUNCH(cdm_gradient_box_u8_kernel<true>, cdm_gradient_box_u8_kernel<false>, kBoxThreads,
                    sizeof(BoxSmem), mod);
-    } else if (pix == 0)
-        SEG_LAUNCH((cdm_gradient_kernel<uint8_t, true>), (cdm_gradient_kernel<uint8_t, false>), kCdmThreads, 0,
-                   gradient_type, mod);
+    } else if (gradient_type == 'r')
+        SEG_LAUNCH(cdm_gradient_r_f32_kernel<true>, cdm_gradient_r_f32_kernel<false>, kFThreads, 0, mod);
+    else if (pix == 0)
+        SEG_LAUNCH((cdm_gradient_d_kernel<uint8_t, true>), (cdm_gradient_d_kernel<uint8_t, false>), kCdmThreads, 0, mod);
     else
-        SEG_LAUNCH((cdm_gradient_kernel<float, true>), (cdm_gradient_kernel<float, false>), kCdmThreads, 0,
-                   gradient_type, mod);
+        SEG_LAUNCH((cdm_gradient_d_kernel<float, true>), (cdm_gradient_d_kernel<float, false>), kCdmThreads, 0, mod);
     count_launch();
     return cudaGetLastError();
 }
