@@ -223,24 +223,194 @@ __global__ void __launch_bounds__(kCdmThreads) cdm_gradient_d_kernel(const CdmSe
         control_block(S, mod);
 }
 
-// Tiled uint8 'r' gradient.  For integer pixels the regression's window sums
-// (sum Js, sum It, sum Js^2, sum It^2, sum Js*It over the clipped 5^3 window) are
-// exact integers, so they are formed here as separable 5-tap box sums over a
-// shared-memory tile (zero outside the volume, the window size m from the clipped
-// extents) -- the same integers the reference sums voxel by voxel, hence
-// bit-identical results at a fraction of the loads.
-constexpr int kTX = 32, kTY = 4, kTZ = 4, kBoxThreads = 128;
-constexpr int kHX = kTX + 4, kHY = kTY + 4, kHZ = kTZ + 4;
-struct BoxSmem {
-    uint8_t J[kHZ][kHY][kHX];
-    uint8_t I[kHZ][kHY][kHX];
-    int p1[5][kHZ][kHY][kTX];  // x-summed
-    int p2[5][kHZ][kTY][kTX];  // x,y-summed
+// Tiled uint8 'r' gradient.  For integer pixels the regression's window sums (sum Js,
+// sum It, sum Js^2, sum It^2, sum Js*It over the clipped 5^3 window) are exact integers, so
+// they are formed here as separable 5-tap box sums over a tile staged as bytes (zero outside
+// the volume, the window size m from the clipped extents) -- the same integers the
+// reference sums voxel by voxel, hence bit-identical results at a fraction of the work.
+//
+// Along x a thread forms the sums of four neighbours from two words a row with byte dot
+// products, along y it adds a run of 8 rows in registers, and the plane sums of the five
+// quantities go to shared memory as one uint4 a voxel (sum Js and sum It share a word: 125
+// pixels of 255 fit 16 bits); along z each thread slides the window over its (x, y) column.
+// Launches, per-tap byte loads and sums of 32-bit words before, so after: 157x189x155 236 / 99
+// us, 91x109x91 58.7 / 33.5, 46x55x46 17.8 / 14.7, 23x28x23 15.8 / 9.8.
+constexpr int kUX = 32, kUY = 8, kUThreads = 256;
+constexpr int kUHX = 40, kUHY = kUY + 4;  // staged rows: 36 bytes used
+struct WinSum {
+    uint32_t s, xx, yy, xy;  // sum Js | sum It << 16, sum Js^2, sum It^2, sum Js*It
 };
+__device__ __forceinline__ void operator+=(WinSum& a, const WinSum& b)
+{
+    a.s += b.s, a.xx += b.xx, a.yy += b.yy, a.xy += b.xy;
+}
+__device__ __forceinline__ void operator-=(WinSum& a, const WinSum& b)
+{
+    a.s -= b.s, a.xx -= b.xx, a.yy -= b.yy, a.xy -= b.xy;
+}
+
+template <int TZ>
+constexpr int box_smem()  // bytes: both staged tiles, then the plane sums
+{
+    return 2 * (TZ + 4) * kUHY * kUHX + (TZ + 4) * kUY * kUX * 16;
+}
+
+template <int TZ>
+__device__ __forceinline__ double gradient_box_u8(const CdmSeg& S, int blk, int mod, unsigned char* __restrict__ smem)
+{
+    constexpr int HZ = TZ + 4, kRows = HZ * kUHY;
+    static_assert(16 * HZ <= kUThreads && kUX * kUY == kUThreads, "threads of the two passes");
+    uint8_t* const sj = smem;
+    uint8_t* const si = smem + kRows * kUHX;
+    uint4* const sum = reinterpret_cast<uint4*>(smem + 2 * kRows * kUHX);
+    const Dim3 D{S.w, S.h, S.d};
+    const uint8_t* __restrict__ Js = (const uint8_t*)S.Js;
+    const uint8_t* __restrict__ It = (const uint8_t*)S.It[mod];
+    float* __restrict__ nd = S.new_d;
+    const int ntx = (D.w + kUX - 1) / kUX, nty = (D.h + kUY - 1) / kUY, ntz = (D.d + TZ - 1) / TZ;
+    const long long ntiles = (long long)ntx * nty * ntz;
+    const long long wl = D.w, whl = D.wh();
+    const int tid = threadIdx.x, lane = tid & 31;
+    double csum = 0.0;
+    for (long long tile = blk; tile < ntiles; tile += S.nblk) {
+        const int x0 = (int)(tile % ntx) * kUX, y0 = (int)(tile / ntx % nty) * kUY, z0 = (int)(tile / ((long long)ntx * nty)) * TZ;
+        __syncthreads();  // the previous tile's readers are done with the buffers
+        // rows by warps: bytes 0..31 of one row, then the last 4 bytes of 8 rows at a time;
+        // the loads of a thread's rows are in flight together
+        auto stage = [&](int r, int hx, bool on, uint8_t& a, uint8_t& b) {
+            const int gx = x0 + hx - 2, gy = y0 + r % kUHY - 2, gz = z0 + r / kUHY - 2;
+            a = b = 0;
+            if (on && gx >= 0 && gy >= 0 && gz >= 0 && gx < D.w && gy < D.h && gz < D.d) {
+                const long long gi = gz * whl + gy * wl + gx;
+                a = __ldg(Js + gi);
+                b = __ldg(It + gi);
+            }
+        };
+        constexpr int kPer = (kRows + 7) / 8, kTail = (kRows + 63) / 64;
+        constexpr int kBatch = kPer % 9 == 0 ? 9 : kPer;
+        for (int q0 = 0; q0 < kPer; q0 += kBatch) {
+            uint8_t a[kBatch], b[kBatch];
+#pragma unroll
+            for (int q = 0; q < kBatch; ++q) {
+                const int r = (tid >> 5) + 8 * (q0 + q);
+                stage(r, lane, r < kRows, a[q], b[q]);
+            }
+#pragma unroll
+            for (int q = 0; q < kBatch; ++q) {
+                const int r = (tid >> 5) + 8 * (q0 + q);
+                if (r < kRows) {
+                    sj[r * kUHX + lane] = a[q];
+                    si[r * kUHX + lane] = b[q];
+                }
+            }
+        }
+        {
+            uint8_t a[kTail], b[kTail];
+#pragma unroll
+            for (int q = 0; q < kTail; ++q) {
+                const int r = (tid >> 2) + 64 * q;
+                stage(r, kUX + (tid & 3), r < kRows, a[q], b[q]);
+            }
+#pragma unroll
+            for (int q = 0; q < kTail; ++q) {
+                const int r = (tid >> 2) + 64 * q;
+                if (r < kRows) {
+                    sj[r * kUHX + kUX + (tid & 3)] = a[q];
+                    si[r * kUHX + kUX + (tid & 3)] = b[q];
+                }
+            }
+        }
+        __syncthreads();
+        if (tid < 16 * HZ) {
+            // x and y sums: 4 voxels in x, 4 in y (8 rows) of plane zz
+            const int quad = tid & 7, half = (tid >> 3) & 1, zz = tid >> 4;
+            const int o = (zz * kUHY + 4 * half) * kUHX + 4 * quad;
+            WinSum row[8][4];
+#pragma unroll
+            for (int r = 0; r < 8; ++r) {
+                const uint32_t* pj = reinterpret_cast<const uint32_t*>(sj + o + r * kUHX);
+                const uint32_t* pi = reinterpret_cast<const uint32_t*>(si + o + r * kUHX);
+                const uint32_t j0 = pj[0], j1 = pj[1], t0 = pi[0], t1 = pi[1];
+#pragma unroll
+                for (int v = 0; v < 4; ++v) {
+                    // bytes v .. v + 3 and v + 4
+                    const uint32_t ja = __funnelshift_r(j0, j1, 8 * v), ta = __funnelshift_r(t0, t1, 8 * v);
+                    const uint32_t jb = (j1 >> (8 * v)) & 0xffu, tb = (t1 >> (8 * v)) & 0xffu;
+                    row[r][v].s = __dp4a(ja, 0x01010101u, jb) + (__dp4a(ta, 0x01010101u, tb) << 16);
+                    row[r][v].xx = __dp4a(ja, ja, jb * jb);
+                    row[r][v].yy = __dp4a(ta, ta, tb * tb);
+                    row[r][v].xy = __dp4a(ja, ta, jb * tb);
+                }
+            }
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+                WinSum w = row[0][v];
+#pragma unroll
+                for (int r = 1; r < 5; ++r)
+                    w += row[r][v];
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    sum[(zz * kUY + 4 * half + r) * kUX + 4 * quad + v] = make_uint4(w.s, w.xx, w.yy, w.xy);
+                    if (r < 3) {
+                        w += row[r + 5][v];
+                        w -= row[r][v];
+                    }
+                }
+            }
+        }
+        __syncthreads();
+        const int xo = lane, yo = tid >> 5, x = x0 + xo, y = y0 + yo;
+        if (x >= D.w || y >= D.h)
+            continue;
+        const int mxy = (min(D.w - 1, x + 2) - max(0, x - 2) + 1) * (min(D.h - 1, y + 2) - max(0, y - 2) + 1);
+        auto plane = [&](int z) {
+            const uint4 q = sum[(z * kUY + yo) * kUX + xo];
+            return WinSum{q.x, q.y, q.z, q.w};
+        };
+        WinSum w = plane(0);
+#pragma unroll
+        for (int z = 1; z < 4; ++z)
+            w += plane(z);
+#pragma unroll 1
+        for (int zo = 0; zo < TZ; ++zo) {
+            const int z = z0 + zo;
+            if (z >= D.d)
+                break;
+            w += plane(zo + 4);
+            const uint8_t* const pj = sj + ((zo + 2) * kUHY + yo + 2) * kUHX + xo + 2;
+            const int js = *pj, it = si[pj - sj];
+            float3 out = make_float3(0.0f, 0.0f, 0.0f);
+            if (!(js == 0 || it == 0)) {
+                const int m = mxy * (min(D.d - 1, z + 2) - max(0, z - 2) + 1);
+                Reg r;
+                regress_finish((double)(int)(w.s & 0xffffu), (double)(int)(w.s >> 16), (double)(int)w.xx,
+                               (double)(int)w.yy, (double)(int)w.xy, m, r);
+                if (r.a > 0.0f) {
+                    // gradient_at from the tile (neighbours are inside the halo)
+                    float3 g;
+                    g.x = (x + 1 < D.w && x) ? (float)((int)pj[1] - (int)pj[-1]) : 0.0f;
+                    g.y = (y + 1 < D.h && y) ? (float)((int)pj[kUHX] - (int)pj[-kUHX]) : 0.0f;
+                    g.z = (z + 1 < D.d && z) ? (float)((int)pj[kUHX * kUHY] - (int)pj[-kUHX * kUHY]) : 0.0f;
+                    const float sc = r.r2 * ((float)js * r.a + r.b - (float)it);
+                    g.x *= sc;
+                    g.y *= sc;
+                    g.z *= sc;
+                    out.x = 0.0f + g.x;
+                    out.y = 0.0f + g.y;
+                    out.z = 0.0f + g.z;
+                    csum += (double)-r.r2;
+                }
+            }
+            store_term(nd, z * whl + y * wl + x, out, mod);
+            w -= plane(zo);
+        }
+    }
+    return csum;
+}
 
 template <bool MULTI>
-__global__ void __launch_bounds__(kBoxThreads) cdm_gradient_box_u8_kernel(const CdmSeg* __restrict__ segs, int nseg,
-                                                                                    int mod)
+__global__ void __launch_bounds__(kUThreads) cdm_gradient_box_u8_kernel(const CdmSeg* __restrict__ segs, int nseg,
+                                                                         int mod)
 {
     const CdmSeg& S = segs[MULTI ? seg_of_block(segs, nseg) : 0];
     const int blk = (int)blockIdx.x - (MULTI ? S.blk0 : 0);
@@ -249,108 +419,12 @@ __global__ void __launch_bounds__(kBoxThreads) cdm_gradient_box_u8_kernel(const 
     if (S.ctl->done || mod >= max(S.nmod, 1))
         return;
     extern __shared__ __align__(16) unsigned char smraw[];
-    BoxSmem& sm = *reinterpret_cast<BoxSmem*>(smraw);
-    const Dim3 D{S.w, S.h, S.d};
-    const uint8_t* __restrict__ Js = (const uint8_t*)S.Js;
-    const uint8_t* __restrict__ It = (const uint8_t*)S.It[mod];
-    float* __restrict__ nd = S.new_d;
-    const int ntx = (D.w + kTX - 1) / kTX, nty = (D.h + kTY - 1) / kTY, ntz = (D.d + kTZ - 1) / kTZ;
-    const int ntiles = ntx * nty * ntz;
-    const long long wl = D.w, whl = D.wh();
-    double csum = 0.0;
-    for (int tile = blk; tile < ntiles; tile += S.nblk) {
-        const int tx = tile % ntx, ty = (tile / ntx) % nty, tz = tile / (ntx * nty);
-        const int x0 = tx * kTX, y0 = ty * kTY, z0 = tz * kTZ;
-        __syncthreads();  // the previous tile's readers are done with the buffers
-        for (int k = threadIdx.x; k < kHZ * kHY * kHX; k += blockDim.x) {
-            const int hx = k % kHX, hy = (k / kHX) % kHY, hz = k / (kHX * kHY);
-            const int gx = x0 + hx - 2, gy = y0 + hy - 2, gz = z0 + hz - 2;
-            uint8_t a = 0, b = 0;
-            if (gx >= 0 && gy >= 0 && gz >= 0 && gx < D.w && gy < D.h && gz < D.d) {
-                const long long gi = (gz * whl) + gy * wl + gx;
-                a = Js[gi];
-                b = It[gi];
-            }
-            sm.J[hz][hy][hx] = a;
-            sm.I[hz][hy][hx] = b;
-        }
-        __syncthreads();
-        for (int k = threadIdx.x; k < kHZ * kHY * kTX; k += blockDim.x) {
-            const int xo = k % kTX, hy = (k / kTX) % kHY, hz = k / (kTX * kHY);
-            int s0 = 0, s1 = 0, s2 = 0, s3 = 0, s4 = 0;
-#pragma unroll
-            for (int dx = 0; dx < 5; ++dx) {
-                const int a = sm.J[hz][hy][xo + dx], b = sm.I[hz][hy][xo + dx];
-                s0 += a;
-                s1 += b;
-                s2 += a * a;
-                s3 += b * b;
-                s4 += a * b;
-            }
-            sm.p1[0][hz][hy][xo] = s0;
-            sm.p1[1][hz][hy][xo] = s1;
-            sm.p1[2][hz][hy][xo] = s2;
-            sm.p1[3][hz][hy][xo] = s3;
-            sm.p1[4][hz][hy][xo] = s4;
-        }
-        __syncthreads();
-        for (int k = threadIdx.x; k < kHZ * kTY * kTX; k += blockDim.x) {
-            const int xo = k % kTX, yo = (k / kTX) % kTY, hz = k / (kTX * kTY);
-#pragma unroll
-            for (int c = 0; c < 5; ++c) {
-                int v = 0;
-#pragma unroll
-                for (int dy = 0; dy < 5; ++dy)
-                    v += sm.p1[c][hz][yo + dy][xo];
-                sm.p2[c][hz][yo][xo] = v;
-            }
-        }
-        __syncthreads();
-        for (int k = threadIdx.x; k < kTZ * kTY * kTX; k += blockDim.x) {
-            const int xo = k % kTX, yo = (k / kTX) % kTY, zo = k / (kTX * kTY);
-            const int x = x0 + xo, y = y0 + yo, z = z0 + zo;
-            if (x >= D.w || y >= D.h || z >= D.d)
-                continue;
-            const long long i = (z * whl) + y * wl + x;
-            const int js = sm.J[zo + 2][yo + 2][xo + 2], it = sm.I[zo + 2][yo + 2][xo + 2];
-            float3 out = make_float3(0.0f, 0.0f, 0.0f);
-            float cost = 0.0f;
-            if (!(js == 0 || it == 0)) {
-                int t[5];
-#pragma unroll
-                for (int c = 0; c < 5; ++c) {
-                    int v = 0;
-#pragma unroll
-                    for (int dz = 0; dz < 5; ++dz)
-                        v += sm.p2[c][zo + dz][yo][xo];
-                    t[c] = v;
-                }
-                const int m = (min(D.w - 1, x + 2) - max(0, x - 2) + 1) * (min(D.h - 1, y + 2) - max(0, y - 2) + 1) *
-                              (min(D.d - 1, z + 2) - max(0, z - 2) + 1);
-                Reg r;
-                regress_finish((double)t[0], (double)t[1], (double)t[2], (double)t[3], (double)t[4], m, r);
-                if (r.a > 0.0f) {
-                    // gradient_at from the tile (neighbours are inside the halo)
-                    float3 g;
-                    g.x = (x + 1 < D.w && x) ? (float)((int)sm.J[zo + 2][yo + 2][xo + 3] - (int)sm.J[zo + 2][yo + 2][xo + 1]) : 0.0f;
-                    g.y = (y + 1 < D.h && y) ? (float)((int)sm.J[zo + 2][yo + 3][xo + 2] - (int)sm.J[zo + 2][yo + 1][xo + 2]) : 0.0f;
-                    g.z = (z + 1 < D.d && z) ? (float)((int)sm.J[zo + 3][yo + 2][xo + 2] - (int)sm.J[zo + 1][yo + 2][xo + 2]) : 0.0f;
-                    const float sc = r.r2 * ((float)js * r.a + r.b - (float)it);
-                    g.x *= sc;
-                    g.y *= sc;
-                    g.z *= sc;
-                    out.x = 0.0f + g.x;
-                    out.y = 0.0f + g.y;
-                    out.z = 0.0f + g.z;
-                    cost = -r.r2;
-                }
-            }
-            store_term(nd, i, out, mod);
-            csum += (double)cost;
-        }
-    }
+    // Tiles of 2 planes where tiles of 8 would leave most SMs idle (23x28x23: 9.8 us / 14.0;
+    // 64^3: 20.4 / 18.6)
+    const long long n = (long long)S.w * S.h * S.d;
+    const double cs = n < 200000 ? gradient_box_u8<2>(S, blk, mod, smraw) : gradient_box_u8<8>(S, blk, mod, smraw);
     __shared__ double red[32];
-    csum = block_sum(csum, red);
+    const double csum = block_sum(cs, red);
     if (threadIdx.x == 0)
         S.cost_part[blk] = csum;
     if (last_block_of_segment(S))
@@ -1219,16 +1293,16 @@ cudaError_t launch_cdm_gradient(const CdmSeg* segs, int nseg, int blocks, int pi
         const unsigned long long bit = 1ull << (dev & 63);
         if (!(attr_set.load() & bit)) {
             e = cudaFuncSetAttribute(cdm_gradient_box_u8_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)sizeof(BoxSmem));
+                                     box_smem<8>());
             if (e == cudaSuccess)
                 e = cudaFuncSetAttribute(cdm_gradient_box_u8_kernel<false>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BoxSmem));
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, box_smem<8>());
             if (e != cudaSuccess)
                 return e;
             attr_set.fetch_or(bit);
         }
-        SEG_LAUNCH(cdm_gradient_box_u8_kernel<true>, cdm_gradient_box_u8_kernel<false>, kBoxThreads,
-                   sizeof(BoxSmem), mod);
+        SEG_LAUNCH(cdm_gradient_box_u8_kernel<true>, cdm_gradient_box_u8_kernel<false>, kUThreads,
+                   box_smem<8>(), mod);
     } else if (gradient_type == 'r')
         SEG_LAUNCH(cdm_gradient_r_f32_kernel<true>, cdm_gradient_r_f32_kernel<false>, kFThreads, 0, mod);
     else if (pix == 0)
