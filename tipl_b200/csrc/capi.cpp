@@ -111,10 +111,7 @@ struct OneSeg {
     CdmCtl c{};
     OneSeg(const int* dim, cudaStream_t st)
     {
-        h.w = dim[0];
-        h.h = dim[1];
-        h.d = dim[2];
-        h.nblk = cdm_blocks_for((long long)dim[0] * dim[1] * dim[2]);
+        cdm_set_dims(h, dim[0], dim[1], dim[2]);
         part.alloc(h.nblk, st);
         ctl.alloc(1, st);
         seg.alloc(1, st);
@@ -937,14 +934,17 @@ regb_status regb_cdm_poisson(regb_field* new_d, void* stream)
         const size_t n = nvox(new_d->dim);
         Staged a;
         a.in(new_d->ptr, n * 12, new_d->location, st, true);
-        DevBuf<float> A(3 * n, st), B(3 * n, st);
         OneSeg s(new_d->dim, st);
-        s.h.new_d = (float*)a.d;
+        const size_t np = s.h.planes_floats();
+        DevBuf<float> N(np, st), A(np, st), B(np, st);
+        s.h.new_d = N.p;
         s.h.aux_d = A.p;
         s.h.tmp_d = B.p;
+        s.h.planar = 1;
         s.upload(st);
-        REGB_CK(launch_cdm_poisson(s.seg.p, 1, s.h.nblk, 12, st));
-        REGB_CK(cudaMemcpyAsync(a.d, A.p, n * 12, cudaMemcpyDeviceToDevice, st));
+        REGB_CK(launch_planes_from_xyz((const float*)a.d, s.h, N.p, st));
+        REGB_CK(launch_cdm_poisson(s.seg.p, 1, s.h.pnb, st));
+        REGB_CK(launch_xyz_from_planes(A.p, s.h, (float*)a.d, st));
         a.out(new_d->ptr, st);
         REGB_CK(cudaStreamSynchronize(st));
         return REGB_OK;

@@ -73,11 +73,8 @@ void CdmLevel::init(const void* const* It_, const void* const* Is_, const std::s
     pix = pix_;
     gtypes = gtypes_;
     seg = CdmSeg{};
-    seg.w = w;
-    seg.h = h;
-    seg.d = d;
+    cdm_set_dims(seg, w, h, d);
     const long long n = (long long)w * h * d;
-    seg.nblk = cdm_blocks_for(n);
     seg.nmod = (int)gtypes.size();
     seg.ndim = ndim;
     for (int m = 0; m < seg.nmod; ++m) {
@@ -86,9 +83,11 @@ void CdmLevel::init(const void* const* It_, const void* const* Is_, const std::s
     }
     js.alloc((size_t)n * (pix ? 4 : 1), st);
     cur.alloc(3 * n, st);
-    nd.alloc(3 * n, st);
-    aux.alloc(3 * n, st);
-    tmp.alloc(3 * n, st);
+    const long long np = std::max(3 * n, seg.planes_floats());
+    nd.alloc(seg.planes_floats(), st);
+    aux.alloc(seg.planes_floats(), st);
+    tmp.alloc(np, st);  // the Poisson iterate's planes, then the interleaved accumulated field
+    seg.planar = 1;
     part.alloc(seg.nblk, st);
     ctl.alloc(1, st);
     seg.Js = js.p;
@@ -114,8 +113,8 @@ void CdmLevel::init(const void* const* It_, const void* const* Is_, const std::s
     REGB_CK(cudaStreamSynchronize(st));  // h_ctl / seg are stack-staged: keep the copies ordered before reuse
 }
 
-void launch_iteration(const CdmSeg* d_segs, int nseg, int blocks, int pix, const std::string& gtypes,
-                      cudaStream_t st)
+void launch_iteration(const CdmSeg* d_segs, int nseg, int blocks, int pblocks, int pix, const std::string& gtypes,
+                      cudaStream_t st, bool first)
 {
     // compose and differentiate each modality in turn (reg/cdm.hpp:422-434); the
     // last gradient launch also makes the loop decisions
@@ -123,7 +122,9 @@ void launch_iteration(const CdmSeg* d_segs, int nseg, int blocks, int pix, const
         REGB_CK(launch_cdm_compose(d_segs, nseg, blocks, pix, st, m));
         REGB_CK(launch_cdm_gradient(d_segs, nseg, blocks, pix, gtypes[m], st, m));
     }
-    REGB_CK(launch_cdm_poisson(d_segs, nseg, blocks, 12, st));                    // + best_d copy, theta
+    REGB_CK(launch_cdm_poisson(d_segs, nseg, pblocks, st));  // + best_d copy
+    if (first)
+        REGB_CK(launch_cdm_theta(d_segs, nseg, blocks, st));
     REGB_CK(launch_cdm_accumulate(d_segs, nseg, blocks, st));
     REGB_CK(launch_cdm_smooth(d_segs, nseg, blocks, st));
 }
@@ -133,10 +134,7 @@ void accumulate_displacement_device(const float* dis, float* new_dis, const int*
     // the accumulate pass of a CDM iteration with speed / theta = 1 (an exact scaling)
     const long long n = (long long)dim[0] * dim[1] * dim[2];
     CdmSeg seg{};
-    seg.w = dim[0];
-    seg.h = dim[1];
-    seg.d = dim[2];
-    seg.nblk = cdm_blocks_for(n);
+    cdm_set_dims(seg, dim[0], dim[1], dim[2]);
     CdmCtl c;
     std::memset(&c, 0, sizeof(c));
     c.scale = 1.0f;
@@ -259,15 +257,17 @@ regb_status cdm_register_multi(const void* const* d_It, const void* const* d_Is,
                 status = REGB_CANCELLED;
         }
         if (!sched) {
-            // kIters iterations per graph launch; the loop decisions live on the
-            // device, so iterations launched after the loop has ended are no-ops
+            // the first iteration (with its theta pass), then kIters iterations per graph
+            // launch; the loop decisions live on the device, so iterations launched after
+            // the loop has ended are no-ops
             constexpr int kIters = 4;
             GraphExec g;
             g.capture([&](cudaStream_t cs) {
                 for (int k = 0; k < kIters; ++k)
-                    launch_iteration(run.d_seg.p, 1, run.seg.nblk, pix, gtypes, cs);
+                    launch_iteration(run.d_seg.p, 1, run.seg.nblk, run.seg.pnb, pix, gtypes, cs, false);
             });
-            for (int it = 0; it < 201; it += kIters) {
+            launch_iteration(run.d_seg.p, 1, run.seg.nblk, run.seg.pnb, pix, gtypes, st, true);
+            for (int it = 1; it < 201; it += kIters) {
                 if (terminated && *terminated) {
                     status = REGB_CANCELLED;
                     break;

@@ -5,11 +5,13 @@
 //
 // One iteration of a level (reg/cdm.hpp:418-470) is the launch sequence
 //   compose -> gradient (+ loop decisions in its last block) -> 12 Poisson sweeps
-//   (the first also saves/restores best_d, the last forms theta) -> accumulate -> smooth
+//   (the first also saves/restores best_d) -> theta, on a level's first iteration only ->
+//   accumulate -> smooth
 // The reference's host-side decisions (cost bookkeeping, cdm_improved, the
 // smoothing schedule, best_d save/restore, theta, the iteration cap) run on the
 // device against CdmCtl, so a level runs without any host round trip; every
 // kernel of an iteration reads ctl->done and returns once a level has left its loop.
+#include <algorithm>
 #include <atomic>
 #include <cfloat>
 #include "common.cuh"
@@ -31,6 +33,8 @@ int cdm_blocks_for(long long nvox)
 // whose blk0 <= blockIdx.x.  Every warp finds it on its own with one ballot per 32
 // entries (all lanes active: this runs first in each kernel); a launch of one entry
 // reads nothing to find it.
+// POISSON: by the Poisson launches' numbering (pblk0).
+template <bool POISSON = false>
 __device__ __forceinline__ int seg_of_block(const CdmSeg* __restrict__ segs, int nseg)
 {
     if (nseg <= 1)
@@ -39,7 +43,7 @@ __device__ __forceinline__ int seg_of_block(const CdmSeg* __restrict__ segs, int
     int k = 0;
     for (int base = 0; base < nseg; base += 32) {
         const int i = base + lane;
-        const unsigned m = __ballot_sync(0xffffffffu, i < nseg && segs[i].blk0 <= b);
+        const unsigned m = __ballot_sync(0xffffffffu, i < nseg && (POISSON ? segs[i].pblk0 : segs[i].blk0) <= b);
         k += __popc(m);
         if (m != 0xffffffffu)
             break;
@@ -117,6 +121,21 @@ __global__ void __launch_bounds__(kCdmThreads) cdm_compose_kernel(const CdmSeg* 
 __device__ void control_block(const CdmSeg& S, int mod);
 __device__ __forceinline__ bool last_block_of_segment(const CdmSeg& S);
 
+// Where voxel i's x component sits in the update field (new_d, aux_d): component planes of
+// padded rows, or interleaved xyz; y and z follow at a stride of update_comp.
+__device__ __forceinline__ long long update_index(const CdmSeg& S, long long i)
+{
+    if (!S.planar)
+        return 3 * i;
+    return i + (long long)((unsigned)i / (unsigned)S.w) * (S.ppitch - S.w);
+}
+// the same of voxel x of row r = z * h + y
+__device__ __forceinline__ long long update_index(const CdmSeg& S, long long r, int x)
+{
+    return S.planar ? r * S.ppitch + x : 3 * (r * S.w + x);
+}
+__device__ __forceinline__ long long update_comp(const CdmSeg& S) { return S.planar ? S.pplane : 1; }
+
 // ------------------------------------------------------------------ gradient
 // x / m rounded like the division, for the window sizes m <= 125 and r = RN(1 / m): the
 // quotient from the reciprocal, corrected twice by its exact remainder.  With r correctly
@@ -178,18 +197,18 @@ __device__ __forceinline__ float3 grad_at(const T* __restrict__ I, const Dim3& D
     return g;
 }
 
-// Stores modality mod's gradient term dd = 0 + g: new_d = dd for the first modality,
-// new_d += dd for the others (reg/cdm.hpp:430-433).
-__device__ __forceinline__ void store_term(float* __restrict__ nd, long long i, float3 out, int mod)
+// Stores modality mod's gradient term dd = 0 + g at q, its components cs apart: new_d = dd
+// for the first modality, new_d += dd for the others (reg/cdm.hpp:430-433).
+__device__ __forceinline__ void store_term(float* __restrict__ q, long long cs, float3 out, int mod)
 {
     if (mod) {
-        out.x = nd[3 * i] + out.x;
-        out.y = nd[3 * i + 1] + out.y;
-        out.z = nd[3 * i + 2] + out.z;
+        out.x = q[0] + out.x;
+        out.y = q[cs] + out.y;
+        out.z = q[2 * cs] + out.z;
     }
-    nd[3 * i] = out.x;
-    nd[3 * i + 1] = out.y;
-    nd[3 * i + 2] = out.z;
+    q[0] = out.x;
+    q[cs] = out.y;
+    q[2 * cs] = out.z;
 }
 
 // cdm_get_gradient_d_imp (reg/cdm.hpp:46-78) of modality mod: the term is 0 + gradient
@@ -212,7 +231,7 @@ __global__ void __launch_bounds__(kCdmThreads) cdm_gradient_d_kernel(const CdmSe
         g.x *= dif;
         g.y *= dif;
         g.z *= dif;
-        store_term(nd, i, make_float3(0.0f + g.x, 0.0f + g.y, 0.0f + g.z), mod);
+        store_term(nd + update_index(S, i), update_comp(S), make_float3(0.0f + g.x, 0.0f + g.y, 0.0f + g.z), mod);
         csum += (double)(dif * dif);
     }
     __shared__ double red[32];
@@ -401,7 +420,7 @@ __device__ __forceinline__ double gradient_box_u8(const CdmSeg& S, int blk, int 
                     csum += (double)-r.r2;
                 }
             }
-            store_term(nd, z * whl + y * wl + x, out, mod);
+            store_term(nd + update_index(S, (long long)z * D.h + y, x), update_comp(S), out, mod);
             w -= plane(zo);
         }
     }
@@ -583,7 +602,7 @@ __device__ __forceinline__ double gradient_r_f32(const CdmSeg& S, int blk, int m
                     csum += (double)-r.r2;
                 }
             }
-            store_term(nd, i0 + v, out, mod);
+            store_term(nd + update_index(S, (long long)z * D.h + y, x), update_comp(S), out, mod);
         }
     }
     return csum;
@@ -751,42 +770,52 @@ __device__ __forceinline__ bool last_block_of_segment(const CdmSeg& S)
 }
 
 // ------------------------------------------------------------------ Poisson
-// cdm_solve_poisson (reg/cdm.hpp:158-253): s0 = new_d * (-1/6); then Jacobi sweeps
+// cdm_solve_poisson (reg/cdm.hpp:158-253): s0 = new_d * (-1/6); then 12 Jacobi sweeps
 // s' = (new_d - s[-1] - s[+1] - s[-w] - s[+w] - s[-wh] - s[+wh]) * (-1/6) with the
 // neighbours taken by flat index, bounds on the flat index only (2-D: -1/4 and no
 // +-wh taps).
-// mode 0: the first sweep, reading s0 = new_d * (-1/6) formed on the fly (the same
-//         float product the reference stores), writing B; it also applies this
-//         iteration's best_d save / restore (reg/cdm.hpp:447-457), which the
-//         reference performs before its Poisson solve -- even on the iteration
-//         that leaves the loop;
-// mode 1: a middle sweep, parity picks A->B or B->A;
-// mode 2: the last sweep (B->A) with the first-iteration max |result| (theta,
-//         reg/cdm.hpp:463-467) formed from the values it writes.
-__device__ __forceinline__ void poisson_point(const float* __restrict__ s, const float* __restrict__ rhs, long long p,
-                                              long long n, long long w, long long wh, bool scale_s, float c6, float* v)
+//
+// The components are planes of their own here, rows padded to 16 bytes (CdmSeg::ppitch).
+// In units of float4 the padded component is a line on which every tap is a fixed offset: a
+// row's ends meet the rows before and after it and a plane's the neighbouring planes, as the
+// flat taps want, except that a row's last voxels may share their float4 with padding.  So
+// the threads of a block take consecutive float4 of a plane whatever rows they belong to, and
+// walk a few planes: the z taps are the thread's registers, x taps too but for a shuffle a
+// side, the rows above and below are loads that the block's walk has just brought to L1.
+// Positions outside the field count as +0, whose subtraction changes nothing, like the taps
+// the reference skips.
+//
+// Bound by L2 (and its latency on small levels): 91x109x91, 12 sweeps replayed by a graph, 137
+// us with a thread per float of the interleaved field (nine scalar loads each, the
+// neighbouring rows and planes from L2), 87 so; 182x218x182 1240 / 613, 46x55x46 49 / 40,
+// 23x28x23 40 / 28.
+constexpr int kPThreads = 256;
+constexpr int kPSweeps = 12;  // reg/cdm.hpp:165
+static_assert(kPSweeps % 2 == 0, "the result lands in aux_d");
+
+// Launch shapes that follow from a level's dims alone.
+void cdm_set_dims(CdmSeg& s, int w, int h, int d)
 {
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        float acc = rhs[3 * p + c];
-        if (scale_s) {
-            if (p >= 1) acc -= s[3 * (p - 1) + c] * c6;
-            if (p < n - 1) acc -= s[3 * (p + 1) + c] * c6;
-            if (p >= w) acc -= s[3 * (p - w) + c] * c6;
-            if (p < n - w) acc -= s[3 * (p + w) + c] * c6;
-            if (p >= wh) acc -= s[3 * (p - wh) + c] * c6;
-            if (p < n - wh) acc -= s[3 * (p + wh) + c] * c6;
-        } else {
-            if (p >= 1) acc -= s[3 * (p - 1) + c];
-            if (p < n - 1) acc -= s[3 * (p + 1) + c];
-            if (p >= w) acc -= s[3 * (p - w) + c];
-            if (p < n - w) acc -= s[3 * (p + w) + c];
-            if (p >= wh) acc -= s[3 * (p - wh) + c];
-            if (p < n - wh) acc -= s[3 * (p + wh) + c];
+    s.w = w;
+    s.h = h;
+    s.d = d;
+    s.nblk = cdm_blocks_for((long long)w * h * d);
+    // component planes of new_d / aux_d / tmp_d: rows padded to 4 voxels, unless that costs
+    // memory that counts (very short rows of a huge volume)
+    const long long rows = (long long)h * d, padded = (w + 3LL) / 4 * 4;
+    s.ppitch = (4 * padded <= 5LL * w || padded * rows < (1LL << 24)) ? padded : w;
+    s.pplane = s.ppitch * rows;
+    // Planes a thread walks: 8 reads a plane of the input 1.25 times, but a level needs two
+    // blocks an SM first (91x109x91 solve: 87 us with 8, 92 with 4; 182x218x182: 613 / 646,
+    // 648 with 16).
+    const long long cols = (s.ppitch * h + 3) / 4, tiles = 3 * ((cols + kPThreads - 1) / kPThreads);
+    s.pdz = 1;
+    for (int dz = 8; dz > 1; dz /= 2)
+        if (tiles * ((d + dz - 1) / dz) >= 148 * 2) {
+            s.pdz = dz;
+            break;
         }
-        acc *= c6;
-        v[c] = acc;
-    }
+    s.pnb = (int)(tiles * ((d + s.pdz - 1) / s.pdz));
 }
 
 // inv_d2 = -0.5 / dimension (reg/cdm.hpp:163,175): -1/6 in 3-D, -1/4 in 2-D.  A 2-D
@@ -797,13 +826,100 @@ __device__ __forceinline__ float poisson_weight(const CdmSeg& S)
     return S.ndim == 2 ? -0.5f / 2.0f : -0.5f / 3.0f;
 }
 
-template <bool MULTI>
-__global__ void __launch_bounds__(kCdmThreads) cdm_poisson_kernel(const CdmSeg* __restrict__ segs, int nseg, int mode,
-                                                                  int parity)
+// One block's part of a sweep: float4 column q of a plane, planes [z0, z1).  FIRST: the input
+// is the right-hand side times c6.  EDGE: some tap of the block may lie outside the field.
+template <bool FIRST, bool EDGE>
+__device__ __forceinline__ void poisson_walk(const CdmSeg& S, const float4* __restrict__ in, const float4* __restrict__ rhs,
+                                             float4* __restrict__ out, unsigned q, int z0, int z1)
 {
-    SEG_BEGIN
-    CdmCtl* c = S.ctl;
-    if (mode == 0) {
+    const unsigned P = (unsigned)(S.ppitch / 4), plane = P * (unsigned)S.h, total = plane * (unsigned)S.d;
+    const float c6 = poisson_weight(S);
+    const int rem = S.w & 3, lane = threadIdx.x & 31;
+    const unsigned xq = q % P;
+    const bool on = q < plane, row_end = xq == P - 1;
+    const bool fix1 = row_end && rem == 1, fix2 = row_end && rem == 2, fix3 = row_end && rem == 3;
+    unsigned i = (unsigned)z0 * plane + q;
+    auto at = [&](unsigned k) {
+        float4 f = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (on && (!EDGE || k < total)) {
+            f = __ldg(in + k);
+            if (FIRST)
+                f = make_float4(f.x * c6, f.y * c6, f.z * c6, f.w * c6);
+        }
+        return f;
+    };
+    auto one = [&](long long k) {
+        float f = 0.0f;
+        if (on && (!EDGE || (k >= 0 && k < 4LL * total))) {
+            f = __ldg(reinterpret_cast<const float*>(in) + k);
+            if (FIRST)
+                f *= c6;
+        }
+        return f;
+    };
+    float4 down = at(i - plane), cur = at(i), up = at(i + plane);
+    for (int z = z0; z < z1; ++z, i += plane) {
+        const float4 ya = at(i - P), yb = at(i + P);
+        const float4 b = on ? __ldg(rhs + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        float4 next = up;
+        if (z + 1 < z1)
+            next = at(i + 2 * plane);
+        // a row's last voxel is where the padding begins
+        const float tail = fix1 ? cur.x : fix2 ? cur.y : fix3 ? cur.z : cur.w;
+        float xl = __shfl_up_sync(0xffffffffu, tail, 1), xr = __shfl_down_sync(0xffffffffu, cur.x, 1);
+        if (lane == 0)
+            xl = one(4LL * i - 1 - (xq == 0 && rem ? 4 - rem : 0));
+        if (lane == 31 || q + 1 == plane)
+            xr = one(4LL * i + 4);
+        const float n1 = fix1 ? xr : cur.y, n2 = fix2 ? xr : cur.z, n3 = fix3 ? xr : cur.w;
+        float4 v;
+        v.x = ((((((b.x - xl) - n1) - ya.x) - yb.x) - down.x) - up.x) * c6;
+        v.y = ((((((b.y - cur.x) - n2) - ya.y) - yb.y) - down.y) - up.y) * c6;
+        v.z = ((((((b.z - cur.y) - n3) - ya.z) - yb.z) - down.z) - up.z) * c6;
+        v.w = ((((((b.w - cur.z) - xr) - ya.w) - yb.w) - down.w) - up.w) * c6;
+        if (on)
+            out[i] = v;
+        down = cur;
+        cur = up;
+        up = next;
+    }
+}
+
+// The part of block b in a sweep over unpadded rows: a float a thread.
+template <bool FIRST>
+__device__ void poisson_flat(const CdmSeg& S, const float* __restrict__ in, const float* __restrict__ rhs,
+                             float* __restrict__ out, long long b, long long blocks)
+{
+    const long long w = S.w, wh = w * S.h, n = wh * S.d;
+    const float c6 = poisson_weight(S);
+    auto at = [&](long long k) { return FIRST ? __ldg(in + k) * c6 : __ldg(in + k); };
+    for (long long p = b * kPThreads + threadIdx.x; p < n; p += blocks * kPThreads) {
+        float acc = __ldg(rhs + p);
+        if (p >= 1) acc -= at(p - 1);
+        if (p < n - 1) acc -= at(p + 1);
+        if (p >= w) acc -= at(p - w);
+        if (p < n - w) acc -= at(p + w);
+        if (p >= wh) acc -= at(p - wh);
+        if (p < n - wh) acc -= at(p + wh);
+        out[p] = acc * c6;
+    }
+}
+
+// One sweep.  FIRST: its input is new_d * (-1/6) formed on the fly (the same float product
+// the reference stores), its output tmp_d; it also applies this iteration's best_d save /
+// restore (reg/cdm.hpp:447-457), which the reference performs before its Poisson solve --
+// even on the iteration that leaves the loop.  Otherwise parity picks aux_d -> tmp_d or
+// tmp_d -> aux_d (the last sweep).
+template <bool FIRST>
+__global__ void __launch_bounds__(kPThreads, 4) cdm_poisson_kernel(const CdmSeg* __restrict__ segs, int nseg, int parity)
+{
+    const CdmSeg& S = segs[nseg > 1 ? seg_of_block<true>(segs, nseg) : 0];
+    const int tile = (int)blockIdx.x - (nseg > 1 ? S.pblk0 : 0);
+    if (tile >= S.pnb)
+        return;
+    const CdmCtl* c = S.ctl;
+    if (FIRST) {
+        const long long n3 = 3LL * S.w * S.h * S.d;
         const float* src = nullptr;
         float* dst = nullptr;
         if (c->save_best) {
@@ -814,84 +930,73 @@ __global__ void __launch_bounds__(kCdmThreads) cdm_poisson_kernel(const CdmSeg* 
             dst = S.cur_d;
         }
         if (dst)
-            for (long long i = first; i < 3 * n; i += stride)
+            for (long long i = (long long)tile * kPThreads + threadIdx.x; i < n3; i += (long long)S.pnb * kPThreads)
                 dst[i] = src[i];
     }
     if (c->done)
         return;
-    const float* __restrict__ rhs = S.new_d;
-    const float* __restrict__ in;
-    float* __restrict__ out;
-    if (mode == 0) {
-        in = rhs;
-        out = S.tmp_d;
-    } else if (mode == 2) {
-        in = S.tmp_d;
-        out = S.aux_d;
-    } else {
-        in = parity ? S.tmp_d : S.aux_d;
-        out = parity ? S.aux_d : S.tmp_d;
-    }
-    const long long w = D.w, wh = D.wh();
-    if (mode != 2) {
-        // one float of the interleaved xyz array per thread: the component's
-        // neighbours at voxel offsets 1, w, wh are float offsets 3, 3w, 3wh, and
-        // the reference's flat-index bounds p >= k / p < n - k are f >= 3k / f < 3(n - k)
-        // -- every tap is a coalesced load, the arithmetic per component unchanged
-        const float c6 = poisson_weight(S);
-        const long long N3 = 3 * n, w3 = 3 * w, wh3 = 3 * wh;
-        const bool sc = (mode == 0);
-        for (long long f = first; f < N3; f += stride) {
-            float acc = rhs[f];
-            if (sc) {
-                if (f >= 3) acc -= in[f - 3] * c6;
-                if (f < N3 - 3) acc -= in[f + 3] * c6;
-                if (f >= w3) acc -= in[f - w3] * c6;
-                if (f < N3 - w3) acc -= in[f + w3] * c6;
-                if (f >= wh3) acc -= in[f - wh3] * c6;
-                if (f < N3 - wh3) acc -= in[f + wh3] * c6;
-            } else {
-                if (f >= 3) acc -= in[f - 3];
-                if (f < N3 - 3) acc -= in[f + 3];
-                if (f >= w3) acc -= in[f - w3];
-                if (f < N3 - w3) acc -= in[f + w3];
-                if (f >= wh3) acc -= in[f - wh3];
-                if (f < N3 - wh3) acc -= in[f + wh3];
-            }
-            acc *= c6;
-            out[f] = acc;
-        }
+    // component slowest, then z chunks: the blocks in flight share planes
+    const int per = S.pnb / 3, comp = tile / per, t = tile % per;
+    const float* const rhs = S.new_d + comp * S.pplane;
+    const float* const in = FIRST ? rhs : (parity ? S.tmp_d : S.aux_d) + comp * S.pplane;
+    float* const out = (FIRST || !parity ? S.tmp_d : S.aux_d) + comp * S.pplane;
+    if (S.ppitch & 3) {
+        poisson_flat<FIRST>(S, in, rhs, out, t, per);
         return;
     }
-    const bool want_theta = (c->theta == 0.0f);
-    float m = 0.0f;
-    for (long long p = first; p < n; p += stride) {
-        float v[3];
-        poisson_point(in, rhs, p, n, w, wh, mode == 0, poisson_weight(S), v);
-        out[3 * p] = v[0];
-        out[3 * p + 1] = v[1];
-        out[3 * p + 2] = v[2];
-        if (want_theta) {
-            // cdm_max_displacement_length: sqrt(double(x*x + y*y + z*z)) as float
-            const float l2 = v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
-            m = fmaxf(m, (float)sqrt((double)l2));
-        }
-    }
-    if (!want_theta)
-        return;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-        m = fmaxf(m, __shfl_down_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0)
-        atomicMax(&c->theta_bits, __float_as_uint(m));
-    if (!last_block_of_segment(S) || threadIdx.x != 0)
-        return;
-    const float theta = __uint_as_float(atomicAdd(&c->theta_bits, 0u));
-    c->theta = theta;
-    if (theta == 0.0f)
-        c->done = 1;
+    const int nz = (S.d + S.pdz - 1) / S.pdz, nq = per / nz;
+    const int z0 = t / nq * S.pdz, z1 = min(S.d, z0 + S.pdz);
+    const unsigned q = (unsigned)(t % nq) * kPThreads + threadIdx.x;
+    const float4* const in4 = reinterpret_cast<const float4*>(in);
+    const float4* const rhs4 = reinterpret_cast<const float4*>(rhs);
+    float4* const out4 = reinterpret_cast<float4*>(out);
+    if (z0 == 0 || z1 == S.d)  // (a plane below and above covers the rows and voxels beside)
+        poisson_walk<FIRST, true>(S, in4, rhs4, out4, q, z0, z1);
     else
-        c->scale = c->speed / theta;
+        poisson_walk<FIRST, false>(S, in4, rhs4, out4, q, z0, z1);
+}
+
+// An interleaved xyz field to the component planes of a segment's scratch, and back.
+__global__ void __launch_bounds__(kCdmThreads) planes_from_xyz_kernel(const float* __restrict__ xyz, Dim3 D,
+                                                                      long long pitch, long long plane,
+                                                                      float* __restrict__ planes)
+{
+    const long long n = D.n();
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+        const long long r = i / D.w, o = r * pitch + (i - r * D.w);
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+            planes[o + c * plane] = __ldg(xyz + 3 * i + c);
+    }
+}
+
+__global__ void __launch_bounds__(kCdmThreads) xyz_from_planes_kernel(const float* __restrict__ planes, Dim3 D,
+                                                                      long long pitch, long long plane,
+                                                                      float* __restrict__ xyz)
+{
+    const long long n = D.n();
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+        const long long r = i / D.w, o = r * pitch + (i - r * D.w);
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+            xyz[3 * i + c] = __ldg(planes + o + c * plane);
+    }
+}
+
+cudaError_t launch_planes_from_xyz(const float* xyz, const CdmSeg& s, float* planes, cudaStream_t st)
+{
+    planes_from_xyz_kernel<<<cdm_blocks_for((long long)s.w * s.h * s.d), kCdmThreads, 0, st>>>(
+        xyz, Dim3{s.w, s.h, s.d}, s.ppitch, s.pplane, planes);
+    count_launch();
+    return cudaGetLastError();
+}
+
+cudaError_t launch_xyz_from_planes(const float* planes, const CdmSeg& s, float* xyz, cudaStream_t st)
+{
+    xyz_from_planes_kernel<<<cdm_blocks_for((long long)s.w * s.h * s.d), kCdmThreads, 0, st>>>(
+        planes, Dim3{s.w, s.h, s.d}, s.ppitch, s.pplane, xyz);
+    count_launch();
+    return cudaGetLastError();
 }
 
 // ------------------------------------------------------------------ theta
@@ -906,9 +1011,11 @@ __global__ void __launch_bounds__(kCdmThreads) cdm_theta_kernel(const CdmSeg* __
     if (c->done || c->theta != 0.0f)
         return;
     const float* __restrict__ d = S.aux_d;
+    const long long cs = update_comp(S);
     float m = 0.0f;
     for (long long i = first; i < n; i += stride) {
-        const float x = d[3 * i], y = d[3 * i + 1], z = d[3 * i + 2];
+        const long long o = update_index(S, i);
+        const float x = d[o], y = d[o + cs], z = d[o + 2 * cs];
         const float l2 = x * x + y * y + z * z;
         const float l = (float)sqrt((double)l2);
         m = fmaxf(m, l);
@@ -942,13 +1049,15 @@ __global__ void __launch_bounds__(kCdmThreads) cdm_accumulate_kernel(const CdmSe
         return;
     const float scale = c->scale;
     const float* __restrict__ nd = S.aux_d;
+    const long long cs = update_comp(S);
     const float* __restrict__ cd = S.cur_d;
     float* __restrict__ out = S.tmp_d;
     const int w = D.w, wh = D.wh();
     if (S.ndim == 2) {
         // the 2-D form: bilinear sample of the mapping cur_d + (x, y); z stays 0
         for (long long i = first; i < n; i += stride) {
-            float dx = nd[3 * i] * scale, dy = nd[3 * i + 1] * scale;
+            const long long o = update_index(S, i);
+            float dx = nd[o] * scale, dy = nd[o + cs] * scale;
             const int x = (int)(i % w), y = (int)(i / w);
             bool ok = false;
             if (dx != 0.0f || dy != 0.0f) {
@@ -988,7 +1097,8 @@ __global__ void __launch_bounds__(kCdmThreads) cdm_accumulate_kernel(const CdmSe
         return;
     }
     for (long long i = first; i < n; i += stride) {
-        float dx = nd[3 * i] * scale, dy = nd[3 * i + 1] * scale, dz = nd[3 * i + 2] * scale;
+        const long long o = update_index(S, i);
+        float dx = nd[o] * scale, dy = nd[o + cs] * scale, dz = nd[o + 2 * cs] * scale;
         int x, y, z;
         unflat((int)i, D, x, y, z);
         bool ok = false;
@@ -1313,14 +1423,12 @@ cudaError_t launch_cdm_gradient(const CdmSeg* segs, int nseg, int blocks, int pi
     return cudaGetLastError();
 }
 
-cudaError_t launch_cdm_poisson(const CdmSeg* segs, int nseg, int blocks, int sweeps, cudaStream_t st)
+cudaError_t launch_cdm_poisson(const CdmSeg* segs, int nseg, int blocks, cudaStream_t st)
 {
-    // sweeps is 12 (reg/cdm.hpp:165): first (B), 10 middle (B->A, A->B, ...), last (B->A)
-    SEG_LAUNCH(cdm_poisson_kernel<true>, cdm_poisson_kernel<false>, kCdmThreads, 0, 0, 0);
-    for (int k = 1; k < sweeps - 1; ++k)
-        SEG_LAUNCH(cdm_poisson_kernel<true>, cdm_poisson_kernel<false>, kCdmThreads, 0, 1, k & 1);
-    SEG_LAUNCH(cdm_poisson_kernel<true>, cdm_poisson_kernel<false>, kCdmThreads, 0, 2, 1);
-    count_launch(sweeps);
+    cdm_poisson_kernel<true><<<blocks, kPThreads, 0, st>>>(segs, nseg, 0);
+    for (int k = 1; k < kPSweeps; ++k)
+        cdm_poisson_kernel<false><<<blocks, kPThreads, 0, st>>>(segs, nseg, k & 1);
+    count_launch(kPSweeps);
     return cudaGetLastError();
 }
 

@@ -85,16 +85,27 @@ struct CdmSeg {
     void* Js;         // composed subject (scratch, pixel type)
     float* cur_d;     // current field
     float* best_d;    // best field
-    float* new_d;     // gradient -> Poisson result (scratch)
+    float* new_d;     // gradient (scratch)
     float* aux_d;     // Poisson iterate A / Poisson result (scratch)
-    float* tmp_d;     // Poisson iterate B / accumulated field (scratch)
+    float* tmp_d;     // Poisson iterate B / accumulated field, interleaved (scratch)
     double* cost_part;  // per-block partial cost sums (nblk entries)
     CdmCtl* ctl;
     // A launch over several segments (their entries back to back) has sum(nblk) blocks:
     // this segment owns blocks [blk0, blk0 + nblk), blk0 ascending along the entries
     // (0 for a launch of this segment alone).
     int blk0;
+    // The Poisson launches' own grid: pnb blocks, pdz planes a thread; pblk0 numbers them as
+    // blk0 does.
+    int pblk0, pnb, pdz;
+    // planar: the update field (new_d, aux_d and the Poisson iterates in tmp_d) is held as
+    // component planes of pplane floats, rows ppitch apart, as the Poisson launches take
+    // it; else interleaved xyz
+    int planar;
+    long long ppitch, pplane;
+    long long planes_floats() const { return 3 * pplane; }
 };
+// Sets a segment's dims and the launch shapes that follow from them.
+void cdm_set_dims(CdmSeg& s, int w, int h, int d);
 
 template <typename T>
 cudaError_t launch_resample(const T* from, Dim3 fd, T* to, Dim3 td, const float* Tm, const int* shift,
@@ -133,11 +144,16 @@ cudaError_t launch_fixed_stats(const uint8_t* f, long long n, int32_t* hist, uns
 cudaError_t launch_cdm_compose(const CdmSeg* segs, int nseg, int blocks, int pix, cudaStream_t st, int mod = 0);
 cudaError_t launch_cdm_gradient(const CdmSeg* segs, int nseg, int blocks, int pix, int gradient_type,
                                 cudaStream_t st, int mod = 0);
-// 12 sweeps; the first also applies best_d save/restore, the last forms theta.
-cudaError_t launch_cdm_poisson(const CdmSeg* segs, int nseg, int blocks, int sweeps, cudaStream_t st);
+// 12 sweeps of planar segments; the first launch also applies best_d save/restore.
+// blocks: sum(pnb) over the entries.
+cudaError_t launch_cdm_poisson(const CdmSeg* segs, int nseg, int blocks, cudaStream_t st);
 cudaError_t launch_cdm_theta(const CdmSeg* segs, int nseg, int blocks, cudaStream_t st);
 cudaError_t launch_cdm_accumulate(const CdmSeg* segs, int nseg, int blocks, cudaStream_t st);
 cudaError_t launch_cdm_smooth(const CdmSeg* segs, int nseg, int blocks, cudaStream_t st);
+
+// An interleaved field to the component planes of s and back.
+cudaError_t launch_planes_from_xyz(const float* xyz, const CdmSeg& s, float* planes, cudaStream_t st);
+cudaError_t launch_xyz_from_planes(const float* planes, const CdmSeg& s, float* xyz, cudaStream_t st);
 
 // Pyramid passes (single volume, device pointers).
 cudaError_t launch_downsample(const void* in, void* out, int w, int h, int d, int pix, cudaStream_t st);

@@ -49,6 +49,7 @@ private:
         CdmLevel* lvl;
         volatile const int* term;
         bool done = false;
+        bool started = false;  // some round has run its first iteration
     };
     void loop();
     std::mutex m_;
