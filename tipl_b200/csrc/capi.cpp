@@ -120,6 +120,7 @@ struct OneSeg {
         std::memset(&c, 0, sizeof(c));
         c.max_iter = 200;
     }
+    CdmSegs segs() const { return CdmSegs{seg.p, &h, 1, h.nblk, h.pnb}; }
     void upload(cudaStream_t st)
     {
         REGB_CK(cudaMemcpyAsync(ctl.p, &c, sizeof(c), cudaMemcpyHostToDevice, st));
@@ -708,7 +709,7 @@ regb_status regb_compose_displacement(const regb_volume* from, const regb_field*
         s.h.cur_d = (float*)f.d;
         s.h.Js = o.d;
         s.upload(st);
-        REGB_CK(launch_cdm_compose(s.seg.p, 1, s.h.nblk, pix_of(from->dtype), st));
+        REGB_CK(launch_cdm_compose(s.segs(), pix_of(from->dtype), st));
         o.out(to->ptr, st);
         REGB_CK(cudaStreamSynchronize(st));
         return REGB_OK;
@@ -846,7 +847,7 @@ regb_status regb_accumulate_displacement(const regb_field* dis, regb_field* new_
         s.h.tmp_d = out.p;
         s.c.scale = 1.0f;
         s.upload(st);
-        REGB_CK(launch_cdm_accumulate(s.seg.p, 1, s.h.nblk, st));
+        REGB_CK(launch_cdm_accumulate(s.segs(), st));
         REGB_CK(cudaMemcpyAsync(b.d, out.p, n * 12, cudaMemcpyDeviceToDevice, st));
         b.out(new_dis->ptr, st);
         REGB_CK(cudaStreamSynchronize(st));
@@ -913,7 +914,7 @@ regb_status regb_cdm_gradient(const regb_volume* Js, const regb_volume* It, regb
         s.h.It[0] = b.d;
         s.h.new_d = (float*)o.d;
         s.upload(st);
-        REGB_CK(launch_cdm_gradient(s.seg.p, 1, s.h.nblk, pix_of(Js->dtype), gradient_type, st));
+        REGB_CK(launch_cdm_gradient(s.segs(), pix_of(Js->dtype), gradient_type, st));
         DevBuf<float> c(1, st);
         REGB_CK(launch_cost_mean(s.seg.p, 1, c.p, st));
         float hc = 0.0f;
@@ -943,7 +944,7 @@ regb_status regb_cdm_poisson(regb_field* new_d, void* stream)
         s.h.planar = 1;
         s.upload(st);
         REGB_CK(launch_planes_from_xyz((const float*)a.d, s.h, N.p, st));
-        REGB_CK(launch_cdm_poisson(s.seg.p, 1, s.h.pnb, st));
+        REGB_CK(launch_cdm_poisson(s.segs(), st));
         REGB_CK(launch_xyz_from_planes(A.p, s.h, (float*)a.d, st));
         a.out(new_d->ptr, st);
         REGB_CK(cudaStreamSynchronize(st));
@@ -965,7 +966,7 @@ regb_status regb_cdm_max_length(const regb_field* d, float* out, void* stream)
         s.h.aux_d = (float*)a.d;
         s.c.speed = 1.0f;
         s.upload(st);
-        REGB_CK(launch_cdm_theta(s.seg.p, 1, s.h.nblk, st));
+        REGB_CK(launch_cdm_theta(s.segs(), st));
         CdmCtl c;
         REGB_CK(cudaMemcpyAsync(&c, s.ctl.p, sizeof(c), cudaMemcpyDeviceToHost, st));
         REGB_CK(cudaStreamSynchronize(st));
@@ -991,7 +992,7 @@ regb_status regb_cdm_smooth(const regb_field* d, regb_field* dd, float smoothing
         s.h.cur_d = (float*)b.d;
         s.c.cur_smoothing = smoothing;
         s.upload(st);
-        REGB_CK(launch_cdm_smooth(s.seg.p, 1, s.h.nblk, st));
+        REGB_CK(launch_cdm_smooth(s.segs(), st));
         b.out(dd->ptr, st);
         REGB_CK(cudaStreamSynchronize(st));
         return REGB_OK;

@@ -113,20 +113,19 @@ void CdmLevel::init(const void* const* It_, const void* const* Is_, const std::s
     REGB_CK(cudaStreamSynchronize(st));  // h_ctl / seg are stack-staged: keep the copies ordered before reuse
 }
 
-void launch_iteration(const CdmSeg* d_segs, int nseg, int blocks, int pblocks, int pix, const std::string& gtypes,
-                      cudaStream_t st, bool first)
+void launch_iteration(const CdmSegs& L, int pix, const std::string& gtypes, cudaStream_t st, bool first)
 {
     // compose and differentiate each modality in turn (reg/cdm.hpp:422-434); the
     // last gradient launch also makes the loop decisions
     for (int m = 0; m < (int)gtypes.size(); ++m) {
-        REGB_CK(launch_cdm_compose(d_segs, nseg, blocks, pix, st, m));
-        REGB_CK(launch_cdm_gradient(d_segs, nseg, blocks, pix, gtypes[m], st, m));
+        REGB_CK(launch_cdm_compose(L, pix, st, m));
+        REGB_CK(launch_cdm_gradient(L, pix, gtypes[m], st, m));
     }
-    REGB_CK(launch_cdm_poisson(d_segs, nseg, pblocks, st));  // + best_d copy
+    REGB_CK(launch_cdm_poisson(L, st));  // + best_d copy
     if (first)
-        REGB_CK(launch_cdm_theta(d_segs, nseg, blocks, st));
-    REGB_CK(launch_cdm_accumulate(d_segs, nseg, blocks, st));
-    REGB_CK(launch_cdm_smooth(d_segs, nseg, blocks, st));
+        REGB_CK(launch_cdm_theta(L, st));
+    REGB_CK(launch_cdm_accumulate(L, st));
+    REGB_CK(launch_cdm_smooth(L, st));
 }
 
 void accumulate_displacement_device(const float* dis, float* new_dis, const int* dim, cudaStream_t st)
@@ -148,7 +147,7 @@ void accumulate_displacement_device(const float* dis, float* new_dis, const int*
     seg.ctl = ctl.p;
     REGB_CK(cudaMemcpyAsync(ctl.p, &c, sizeof(c), cudaMemcpyHostToDevice, st));
     REGB_CK(cudaMemcpyAsync(d_seg.p, &seg, sizeof(seg), cudaMemcpyHostToDevice, st));
-    REGB_CK(launch_cdm_accumulate(d_seg.p, 1, seg.nblk, st));
+    REGB_CK(launch_cdm_accumulate(CdmSegs{d_seg.p, &seg, 1, seg.nblk, seg.pnb}, st));
     REGB_CK(cudaMemcpyAsync(new_dis, out.p, sizeof(float) * 3 * n, cudaMemcpyDeviceToDevice, st));
     REGB_CK(cudaStreamSynchronize(st));  // c and seg are stack-staged
 }
@@ -261,12 +260,13 @@ regb_status cdm_register_multi(const void* const* d_It, const void* const* d_Is,
             // launch; the loop decisions live on the device, so iterations launched after
             // the loop has ended are no-ops
             constexpr int kIters = 4;
+            const CdmSegs one{run.d_seg.p, &run.seg, 1, run.seg.nblk, run.seg.pnb};
             GraphExec g;
             g.capture([&](cudaStream_t cs) {
                 for (int k = 0; k < kIters; ++k)
-                    launch_iteration(run.d_seg.p, 1, run.seg.nblk, run.seg.pnb, pix, gtypes, cs, false);
+                    launch_iteration(one, pix, gtypes, cs, false);
             });
-            launch_iteration(run.d_seg.p, 1, run.seg.nblk, run.seg.pnb, pix, gtypes, st, true);
+            launch_iteration(one, pix, gtypes, st, true);
             for (int it = 1; it < 201; it += kIters) {
                 if (terminated && *terminated) {
                     status = REGB_CANCELLED;

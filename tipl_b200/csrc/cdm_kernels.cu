@@ -52,9 +52,12 @@ __device__ __forceinline__ int seg_of_block(const CdmSeg* __restrict__ segs, int
 }
 
 // MULTI: the kernel's instantiation for launches over several entries; a launch of one
-// entry takes the other, which has no lookup in its code at all.
+// entry takes the other, which has no lookup in its code at all and the entry as a kernel
+// argument (`one`): a trip to memory less before its first load, 0.3 us of a launch.
+#define SEG_ARGS const CdmSeg *__restrict__ segs, int nseg, const __grid_constant__ CdmSeg one
+#define SEG_OF(poisson) (MULTI ? segs[seg_of_block<poisson>(segs, nseg)] : one)
 #define SEG_BEGIN                                                  \
-    const CdmSeg& S = segs[MULTI ? seg_of_block(segs, nseg) : 0];  \
+    const CdmSeg& S = SEG_OF(false);                               \
     const int blk = (int)blockIdx.x - (MULTI ? S.blk0 : 0);        \
     if (blk >= S.nblk)                                             \
         return;                                                    \
@@ -68,7 +71,7 @@ __device__ __forceinline__ int seg_of_block(const CdmSeg* __restrict__ segs, int
 // displacement is exactly zero, else the trilinear sample at x + d; failed
 // samples are 0.
 template <typename T, bool MULTI>
-__global__ void __launch_bounds__(kCdmThreads) cdm_compose_kernel(const CdmSeg* __restrict__ segs, int nseg, int mod)
+__global__ void __launch_bounds__(kCdmThreads) cdm_compose_kernel(SEG_ARGS, int mod)
 {
     SEG_BEGIN
     if (S.ctl->done || mod >= max(S.nmod, 1))
@@ -214,7 +217,7 @@ __device__ __forceinline__ void store_term(float* __restrict__ q, long long cs, 
 // cdm_get_gradient_d_imp (reg/cdm.hpp:46-78) of modality mod: the term is 0 + gradient
 // term; the cost of every voxel is summed per block in double.
 template <typename T, bool MULTI>
-__global__ void __launch_bounds__(kCdmThreads) cdm_gradient_d_kernel(const CdmSeg* __restrict__ segs, int nseg, int mod)
+__global__ void __launch_bounds__(kCdmThreads) cdm_gradient_d_kernel(SEG_ARGS, int mod)
 {
     SEG_BEGIN
     if (S.ctl->done || mod >= max(S.nmod, 1))
@@ -428,10 +431,10 @@ __device__ __forceinline__ double gradient_box_u8(const CdmSeg& S, int blk, int 
 }
 
 template <bool MULTI>
-__global__ void __launch_bounds__(kUThreads) cdm_gradient_box_u8_kernel(const CdmSeg* __restrict__ segs, int nseg,
+__global__ void __launch_bounds__(kUThreads) cdm_gradient_box_u8_kernel(SEG_ARGS,
                                                                          int mod)
 {
-    const CdmSeg& S = segs[MULTI ? seg_of_block(segs, nseg) : 0];
+    const CdmSeg& S = SEG_OF(false);
     const int blk = (int)blockIdx.x - (MULTI ? S.blk0 : 0);
     if (blk >= S.nblk)
         return;
@@ -609,10 +612,10 @@ __device__ __forceinline__ double gradient_r_f32(const CdmSeg& S, int blk, int m
 }
 
 template <bool MULTI>
-__global__ void __launch_bounds__(kFThreads, 3) cdm_gradient_r_f32_kernel(const CdmSeg* __restrict__ segs, int nseg,
+__global__ void __launch_bounds__(kFThreads, 3) cdm_gradient_r_f32_kernel(SEG_ARGS,
                                                                           int mod)
 {
-    const CdmSeg& S = segs[MULTI ? seg_of_block(segs, nseg) : 0];
+    const CdmSeg& S = SEG_OF(false);
     const int blk = (int)blockIdx.x - (MULTI ? S.blk0 : 0);
     if (blk >= S.nblk)
         return;
@@ -826,11 +829,20 @@ __device__ __forceinline__ float poisson_weight(const CdmSeg& S)
     return S.ndim == 2 ? -0.5f / 2.0f : -0.5f / 3.0f;
 }
 
+// A load the compiler leaves where it stands; zeros where !ok.
+__device__ __forceinline__ float4 load_now(const float4* __restrict__ p, bool ok)
+{
+    float4 f = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (ok)
+        asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(f.x), "=f"(f.y), "=f"(f.z), "=f"(f.w) : "l"(p));
+    return f;
+}
+
 // One block's part of a sweep: float4 column q of a plane, planes [z0, z1).  FIRST: the input
 // is the right-hand side times c6.  EDGE: some tap of the block may lie outside the field.
 template <bool FIRST, bool EDGE>
 __device__ __forceinline__ void poisson_walk(const CdmSeg& S, const float4* __restrict__ in, const float4* __restrict__ rhs,
-                                             float4* __restrict__ out, unsigned q, int z0, int z1)
+                                             float4* __restrict__ out, unsigned q, int z0, int z1, int done)
 {
     const unsigned P = (unsigned)(S.ppitch / 4), plane = P * (unsigned)S.h, total = plane * (unsigned)S.d;
     const float c6 = poisson_weight(S);
@@ -839,14 +851,15 @@ __device__ __forceinline__ void poisson_walk(const CdmSeg& S, const float4* __re
     const bool on = q < plane, row_end = xq == P - 1;
     const bool fix1 = row_end && rem == 1, fix2 = row_end && rem == 2, fix3 = row_end && rem == 3;
     unsigned i = (unsigned)z0 * plane + q;
+    auto inside = [&](unsigned k) { return on && (!EDGE || k < total); };
+    auto value = [&](float4 f, unsigned k) {
+        return FIRST && inside(k) ? make_float4(f.x * c6, f.y * c6, f.z * c6, f.w * c6) : f;
+    };
     auto at = [&](unsigned k) {
         float4 f = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (on && (!EDGE || k < total)) {
+        if (inside(k))
             f = __ldg(in + k);
-            if (FIRST)
-                f = make_float4(f.x * c6, f.y * c6, f.z * c6, f.w * c6);
-        }
-        return f;
+        return value(f, k);
     };
     auto one = [&](long long k) {
         float f = 0.0f;
@@ -857,10 +870,18 @@ __device__ __forceinline__ void poisson_walk(const CdmSeg& S, const float4* __re
         }
         return f;
     };
-    float4 down = at(i - plane), cur = at(i), up = at(i + plane);
+    // the first plane's loads go out before the loop flag is waited for
+    float4 down = load_now(in + (i - plane), inside(i - plane)), cur = load_now(in + i, on),
+           up = load_now(in + (i + plane), inside(i + plane)), b = load_now(rhs + i, on);
+    if (done)
+        return;
+    down = value(down, i - plane);
+    cur = value(cur, i);
+    up = value(up, i + plane);
     for (int z = z0; z < z1; ++z, i += plane) {
         const float4 ya = at(i - P), yb = at(i + P);
-        const float4 b = on ? __ldg(rhs + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (z > z0)
+            b = on ? __ldg(rhs + i) : b;
         float4 next = up;
         if (z + 1 < z1)
             next = at(i + 2 * plane);
@@ -910,15 +931,36 @@ __device__ void poisson_flat(const CdmSeg& S, const float* __restrict__ in, cons
 // restore (reg/cdm.hpp:447-457), which the reference performs before its Poisson solve --
 // even on the iteration that leaves the loop.  Otherwise parity picks aux_d -> tmp_d or
 // tmp_d -> aux_d (the last sweep).
-template <bool FIRST>
-__global__ void __launch_bounds__(kPThreads, 4) cdm_poisson_kernel(const CdmSeg* __restrict__ segs, int nseg, int parity)
+template <bool FIRST, bool MULTI>
+__global__ void __launch_bounds__(kPThreads, 4) cdm_poisson_kernel(SEG_ARGS, int parity)
 {
-    const CdmSeg& S = segs[nseg > 1 ? seg_of_block<true>(segs, nseg) : 0];
-    const int tile = (int)blockIdx.x - (nseg > 1 ? S.pblk0 : 0);
+    const CdmSeg& S = SEG_OF(true);
+    const int tile = (int)blockIdx.x - (MULTI ? S.pblk0 : 0);
     if (tile >= S.pnb)
         return;
     const CdmCtl* c = S.ctl;
-    if (FIRST) {
+    const int done = c->done;
+    // component slowest, then z chunks: the blocks in flight share planes
+    const int per = S.pnb / 3, comp = tile / per, t = tile % per;
+    const float* const rhs = S.new_d + comp * S.pplane;
+    const float* const in = FIRST ? rhs : (parity ? S.tmp_d : S.aux_d) + comp * S.pplane;
+    float* const out = (FIRST || !parity ? S.tmp_d : S.aux_d) + comp * S.pplane;
+    if (S.ppitch & 3) {
+        if (!done)
+            poisson_flat<FIRST>(S, in, rhs, out, t, per);
+    } else {
+        const int nz = (S.d + S.pdz - 1) / S.pdz, nq = per / nz;
+        const int z0 = t / nq * S.pdz, z1 = min(S.d, z0 + S.pdz);
+        const unsigned q = (unsigned)(t % nq) * kPThreads + threadIdx.x;
+        const float4* const in4 = reinterpret_cast<const float4*>(in);
+        const float4* const rhs4 = reinterpret_cast<const float4*>(rhs);
+        float4* const out4 = reinterpret_cast<float4*>(out);
+        if (z0 == 0 || z1 == S.d)  // (a plane below and above covers the rows and voxels beside)
+            poisson_walk<FIRST, true>(S, in4, rhs4, out4, q, z0, z1, done);
+        else
+            poisson_walk<FIRST, false>(S, in4, rhs4, out4, q, z0, z1, done);
+    }
+    if (FIRST) {  // (last: the sweep reads neither field)
         const long long n3 = 3LL * S.w * S.h * S.d;
         const float* src = nullptr;
         float* dst = nullptr;
@@ -933,27 +975,6 @@ __global__ void __launch_bounds__(kPThreads, 4) cdm_poisson_kernel(const CdmSeg*
             for (long long i = (long long)tile * kPThreads + threadIdx.x; i < n3; i += (long long)S.pnb * kPThreads)
                 dst[i] = src[i];
     }
-    if (c->done)
-        return;
-    // component slowest, then z chunks: the blocks in flight share planes
-    const int per = S.pnb / 3, comp = tile / per, t = tile % per;
-    const float* const rhs = S.new_d + comp * S.pplane;
-    const float* const in = FIRST ? rhs : (parity ? S.tmp_d : S.aux_d) + comp * S.pplane;
-    float* const out = (FIRST || !parity ? S.tmp_d : S.aux_d) + comp * S.pplane;
-    if (S.ppitch & 3) {
-        poisson_flat<FIRST>(S, in, rhs, out, t, per);
-        return;
-    }
-    const int nz = (S.d + S.pdz - 1) / S.pdz, nq = per / nz;
-    const int z0 = t / nq * S.pdz, z1 = min(S.d, z0 + S.pdz);
-    const unsigned q = (unsigned)(t % nq) * kPThreads + threadIdx.x;
-    const float4* const in4 = reinterpret_cast<const float4*>(in);
-    const float4* const rhs4 = reinterpret_cast<const float4*>(rhs);
-    float4* const out4 = reinterpret_cast<float4*>(out);
-    if (z0 == 0 || z1 == S.d)  // (a plane below and above covers the rows and voxels beside)
-        poisson_walk<FIRST, true>(S, in4, rhs4, out4, q, z0, z1);
-    else
-        poisson_walk<FIRST, false>(S, in4, rhs4, out4, q, z0, z1);
 }
 
 // An interleaved xyz field to the component planes of a segment's scratch, and back.
@@ -1004,7 +1025,7 @@ cudaError_t launch_xyz_from_planes(const float* planes, const CdmSeg& s, float* 
 // first iteration of a level); the last block sets theta and speed/theta, or
 // leaves the loop when theta is 0 (reg/cdm.hpp:463-467).
 template <bool MULTI>
-__global__ void __launch_bounds__(kCdmThreads) cdm_theta_kernel(const CdmSeg* __restrict__ segs, int nseg)
+__global__ void __launch_bounds__(kCdmThreads) cdm_theta_kernel(SEG_ARGS)
 {
     SEG_BEGIN
     CdmCtl* c = S.ctl;
@@ -1041,7 +1062,7 @@ __global__ void __launch_bounds__(kCdmThreads) cdm_theta_kernel(const CdmSeg* __
 // non-zero and the sample lands inside, else cur_d.  The mapping cur_d + id is
 // formed per corner exactly as displacement_to_mapping stores it.
 template <bool MULTI>
-__global__ void __launch_bounds__(kCdmThreads) cdm_accumulate_kernel(const CdmSeg* __restrict__ segs, int nseg)
+__global__ void __launch_bounds__(kCdmThreads) cdm_accumulate_kernel(SEG_ARGS)
 {
     SEG_BEGIN
     const CdmCtl* c = S.ctl;
@@ -1150,7 +1171,7 @@ __global__ void __launch_bounds__(kCdmThreads) cdm_accumulate_kernel(const CdmSe
 // d[+w] + d[-w] + d[+wh] + d[-wh]) by flat index; s == 0 leaves cur_d as it is.
 // 2-D: s/4 and four neighbours (the +-wh taps of a d == 1 level fall outside).
 template <bool MULTI>
-__global__ void __launch_bounds__(kCdmThreads) cdm_smooth_kernel(const CdmSeg* __restrict__ segs, int nseg)
+__global__ void __launch_bounds__(kCdmThreads) cdm_smooth_kernel(SEG_ARGS)
 {
     SEG_BEGIN
     const CdmCtl* c = S.ctl;
@@ -1366,18 +1387,15 @@ cudaError_t launch_cdm_status(const CdmSeg* segs, int nseg, int* out, cudaStream
 }
 
 // ------------------------------------------------------------------ launchers
-// blocks: the launch's blocks, sum(nblk) over its nseg segment entries (their blk0 set
-// accordingly); one entry alone: its nblk.
-#define SEG_GRID dim3(blocks)
-#define SEG_LAUNCH(multi, single, threads, smem, ...)                                  \
-    do {                                                                               \
-        if (nseg > 1)                                                                  \
-            multi<<<SEG_GRID, threads, smem, st>>>(segs, nseg, ##__VA_ARGS__);         \
-        else                                                                           \
-            single<<<SEG_GRID, threads, smem, st>>>(segs, nseg, ##__VA_ARGS__);        \
+#define SEG_LAUNCH(multi, single, threads, smem, ...)                                      \
+    do {                                                                                   \
+        if (L.n > 1)                                                                       \
+            multi<<<L.blocks, threads, smem, st>>>(L.dev, L.n, *L.host, ##__VA_ARGS__);    \
+        else                                                                               \
+            single<<<L.blocks, threads, smem, st>>>(L.dev, L.n, *L.host, ##__VA_ARGS__);   \
     } while (0)
 
-cudaError_t launch_cdm_compose(const CdmSeg* segs, int nseg, int blocks, int pix, cudaStream_t st, int mod)
+cudaError_t launch_cdm_compose(const CdmSegs& L, int pix, cudaStream_t st, int mod)
 {
     if (mod < 0 || mod >= kCdmMaxModalities)
         return cudaErrorInvalidValue;
@@ -1389,7 +1407,7 @@ cudaError_t launch_cdm_compose(const CdmSeg* segs, int nseg, int blocks, int pix
     return cudaGetLastError();
 }
 
-cudaError_t launch_cdm_gradient(const CdmSeg* segs, int nseg, int blocks, int pix, int gradient_type,
+cudaError_t launch_cdm_gradient(const CdmSegs& L, int pix, int gradient_type,
                                 cudaStream_t st, int mod)
 {
     if (mod < 0 || mod >= kCdmMaxModalities)
@@ -1423,30 +1441,32 @@ cudaError_t launch_cdm_gradient(const CdmSeg* segs, int nseg, int blocks, int pi
     return cudaGetLastError();
 }
 
-cudaError_t launch_cdm_poisson(const CdmSeg* segs, int nseg, int blocks, cudaStream_t st)
+cudaError_t launch_cdm_poisson(const CdmSegs& L, cudaStream_t st)
 {
-    cdm_poisson_kernel<true><<<blocks, kPThreads, 0, st>>>(segs, nseg, 0);
-    for (int k = 1; k < kPSweeps; ++k)
-        cdm_poisson_kernel<false><<<blocks, kPThreads, 0, st>>>(segs, nseg, k & 1);
+    for (int k = 0; k < kPSweeps; ++k) {
+        auto kernel = L.n > 1 ? (k ? cdm_poisson_kernel<false, true> : cdm_poisson_kernel<true, true>)
+                              : (k ? cdm_poisson_kernel<false, false> : cdm_poisson_kernel<true, false>);
+        kernel<<<L.pblocks, kPThreads, 0, st>>>(L.dev, L.n, *L.host, k & 1);
+    }
     count_launch(kPSweeps);
     return cudaGetLastError();
 }
 
-cudaError_t launch_cdm_theta(const CdmSeg* segs, int nseg, int blocks, cudaStream_t st)
+cudaError_t launch_cdm_theta(const CdmSegs& L, cudaStream_t st)
 {
     SEG_LAUNCH(cdm_theta_kernel<true>, cdm_theta_kernel<false>, kCdmThreads, 0);
     count_launch();
     return cudaGetLastError();
 }
 
-cudaError_t launch_cdm_accumulate(const CdmSeg* segs, int nseg, int blocks, cudaStream_t st)
+cudaError_t launch_cdm_accumulate(const CdmSegs& L, cudaStream_t st)
 {
     SEG_LAUNCH(cdm_accumulate_kernel<true>, cdm_accumulate_kernel<false>, kCdmThreads, 0);
     count_launch();
     return cudaGetLastError();
 }
 
-cudaError_t launch_cdm_smooth(const CdmSeg* segs, int nseg, int blocks, cudaStream_t st)
+cudaError_t launch_cdm_smooth(const CdmSegs& L, cudaStream_t st)
 {
     SEG_LAUNCH(cdm_smooth_kernel<true>, cdm_smooth_kernel<false>, kCdmThreads, 0);
     count_launch();

@@ -36,12 +36,9 @@ struct CdmLevel {
               const regb_cdm_param& p, float* best, cudaStream_t st, int ndim = 3);
 };
 
-// One iteration of every segment in d_segs (reg/cdm.hpp:418-470); the segments
-// share pix and the gradient types of their modalities (gtypes, one char each).
-// blocks / pblocks: sum(nblk) / sum(pnb) over the nseg entries, whose blk0 / pblk0
-// number them (one entry alone: its own, numbered from 0).  first: some entry is on its
-// level's first iteration, whose Poisson result sets theta.
-void launch_iteration(const CdmSeg* d_segs, int nseg, int blocks, int pblocks, int pix, const std::string& gtypes,
-                      cudaStream_t st, bool first);
+// One iteration of every segment of L (reg/cdm.hpp:418-470); they share pix and the gradient
+// types of their modalities (gtypes, one char each).  first: some entry is on its level's
+// first iteration, whose Poisson result sets theta.
+void launch_iteration(const CdmSegs& L, int pix, const std::string& gtypes, cudaStream_t st, bool first);
 
 }  // namespace regb

@@ -104,6 +104,14 @@ struct CdmSeg {
     long long ppitch, pplane;
     long long planes_floats() const { return 3 * pplane; }
 };
+// The segments of one launch: n entries on the device and on the host (one entry alone is
+// passed to the kernels by value); blocks / pblocks: sum(nblk) / sum(pnb) over the entries,
+// whose blk0 / pblk0 number them.
+struct CdmSegs {
+    const CdmSeg* dev;
+    const CdmSeg* host;
+    int n, blocks, pblocks;
+};
 // Sets a segment's dims and the launch shapes that follow from them.
 void cdm_set_dims(CdmSeg& s, int w, int h, int d);
 
@@ -135,21 +143,19 @@ int cost_blocks_per_sm(bool is_corr);
 cudaError_t launch_fixed_stats(const uint8_t* f, long long n, int32_t* hist, unsigned long long* sums,
                                cudaStream_t st);
 
-// CDM passes.  pix: 0 = uint8, 1 = float.  segs is a device array of nseg segments;
-// blocks is gridDim.x per segment.
+// CDM passes.  pix: 0 = uint8, 1 = float.
 // mod selects the modality pair: compose reads Is[mod]; the gradient reads It[mod],
 // writes new_d for modality 0 and adds to it for the others, and its last block keeps
 // the modality's mean cost; after the last modality that block also runs the loop
 // decisions.
-cudaError_t launch_cdm_compose(const CdmSeg* segs, int nseg, int blocks, int pix, cudaStream_t st, int mod = 0);
-cudaError_t launch_cdm_gradient(const CdmSeg* segs, int nseg, int blocks, int pix, int gradient_type,
+cudaError_t launch_cdm_compose(const CdmSegs& L, int pix, cudaStream_t st, int mod = 0);
+cudaError_t launch_cdm_gradient(const CdmSegs& L, int pix, int gradient_type,
                                 cudaStream_t st, int mod = 0);
 // 12 sweeps of planar segments; the first launch also applies best_d save/restore.
-// blocks: sum(pnb) over the entries.
-cudaError_t launch_cdm_poisson(const CdmSeg* segs, int nseg, int blocks, cudaStream_t st);
-cudaError_t launch_cdm_theta(const CdmSeg* segs, int nseg, int blocks, cudaStream_t st);
-cudaError_t launch_cdm_accumulate(const CdmSeg* segs, int nseg, int blocks, cudaStream_t st);
-cudaError_t launch_cdm_smooth(const CdmSeg* segs, int nseg, int blocks, cudaStream_t st);
+cudaError_t launch_cdm_poisson(const CdmSegs& L, cudaStream_t st);
+cudaError_t launch_cdm_theta(const CdmSegs& L, cudaStream_t st);
+cudaError_t launch_cdm_accumulate(const CdmSegs& L, cudaStream_t st);
+cudaError_t launch_cdm_smooth(const CdmSegs& L, cudaStream_t st);
 
 // An interleaved field to the component planes of s and back.
 cudaError_t launch_planes_from_xyz(const float* xyz, const CdmSeg& s, float* planes, cudaStream_t st);

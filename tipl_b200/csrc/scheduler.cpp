@@ -110,8 +110,8 @@ void CdmScheduler::loop()
             for (int it = 0; it < iters_; ++it)
                 for (const Group& g : groups) {
                     const Entry* e = cur[order[g.g0]];
-                    launch_iteration(segs_.p + g.g0, g.g1 - g.g0, g.blocks, g.pblocks, e->lvl->pix, e->lvl->gtypes, st_,
-                                     it == 0 && g.first);
+                    launch_iteration(CdmSegs{segs_.p + g.g0, h_segs_.p + g.g0, g.g1 - g.g0, g.blocks, g.pblocks},
+                                     e->lvl->pix, e->lvl->gtypes, st_, it == 0 && g.first);
                 }
             REGB_CK(launch_cdm_status(segs_.p, n, status_.p, st_));
             REGB_CK(cudaMemcpyAsync(h_status_.p, status_.p, sizeof(int) * n, cudaMemcpyDeviceToHost, st_));
