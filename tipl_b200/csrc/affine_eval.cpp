@@ -471,11 +471,21 @@ AffineEvaluator::AffineEvaluator(const std::vector<Pair>& levels, int cost_type,
         L.row_hist.alloc(256, st);
         L.sums.alloc(2, st);
         REGB_CK(launch_fixed_stats(grid, n, L.row_hist.p, L.sums.p, st));
+        if (cost_type != REGB_COST_CORR)
+            continue;  // the row histogram stays on the device: nothing to wait for
         REGB_CK(cudaMemcpyAsync(h.p, L.sums.p, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
         REGB_CK(cudaStreamSynchronize(st));
         L.sx = (long long)h.p[0];
         L.sxx = (long long)h.p[1];
     }
+}
+
+void AffineEvaluator::set_batcher(AffineBatcher* b)
+{
+    // the batcher's streams read what the constructor queued on this one
+    if (b)
+        REGB_CK(cudaStreamSynchronize(st_));
+    batcher_ = b;
 }
 
 void AffineEvaluator::make_task(int level, const float* T, AffineTask& t) const

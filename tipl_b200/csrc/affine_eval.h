@@ -101,7 +101,7 @@ public:
     void make_task(int level, const float* T, AffineTask& out) const;
     int cost_type() const { return cost_type_; }
     // Route evaluations through a cross-job batcher instead of launching directly.
-    void set_batcher(AffineBatcher* b) { batcher_ = b; }
+    void set_batcher(AffineBatcher* b);
 
 private:
     struct Lvl {
