@@ -120,7 +120,7 @@ struct OneSeg {
         std::memset(&c, 0, sizeof(c));
         c.max_iter = 200;
     }
-    CdmSegs segs() const { return CdmSegs{seg.p, &h, 1, h.nblk, h.pnb}; }
+    CdmSegs segs() const { return CdmSegs{seg.p, &h, 1, h.nblk, h.pnb, h.tnb}; }
     void upload(cudaStream_t st)
     {
         REGB_CK(cudaMemcpyAsync(ctl.p, &c, sizeof(c), cudaMemcpyHostToDevice, st));
@@ -706,7 +706,7 @@ regb_status regb_compose_displacement(const regb_volume* from, const regb_field*
         o.in(to->ptr, n * ps, to->location, st, false);
         OneSeg s(from->dim, st);
         s.h.Is[0] = a.d;
-        s.h.cur_d = (float*)f.d;
+        s.h.field[0] = (float*)f.d;
         s.h.Js = o.d;
         s.upload(st);
         REGB_CK(launch_cdm_compose(s.segs(), pix_of(from->dtype), st));
@@ -842,7 +842,7 @@ regb_status regb_accumulate_displacement(const regb_field* dis, regb_field* new_
         b.in(new_dis->ptr, n * 12, new_dis->location, st, true);
         DevBuf<float> out(3 * n, st);
         OneSeg s(dis->dim, st);
-        s.h.cur_d = (float*)a.d;
+        s.h.field[0] = (float*)a.d;
         s.h.aux_d = (float*)b.d;
         s.h.tmp_d = out.p;
         s.c.scale = 1.0f;
@@ -989,7 +989,7 @@ regb_status regb_cdm_smooth(const regb_field* d, regb_field* dd, float smoothing
         b.in(dd->ptr, n * 12, dd->location, st, true);
         OneSeg s(d->dim, st);
         s.h.tmp_d = (float*)a.d;
-        s.h.cur_d = (float*)b.d;
+        s.h.field[0] = (float*)b.d;
         s.c.cur_smoothing = smoothing;
         s.upload(st);
         REGB_CK(launch_cdm_smooth(s.segs(), st));

@@ -68,7 +68,7 @@ void GraphExec::reset()
 }
 
 void CdmLevel::init(const void* const* It_, const void* const* Is_, const std::string& gtypes_, int w, int h, int d,
-                    int pix_, const regb_cdm_param& p, float* best, cudaStream_t st, int ndim)
+                    int pix_, const regb_cdm_param& p, const float* best, cudaStream_t st, int ndim)
 {
     pix = pix_;
     gtypes = gtypes_;
@@ -82,17 +82,17 @@ void CdmLevel::init(const void* const* It_, const void* const* Is_, const std::s
         seg.Is[m] = Is_[m];
     }
     js.alloc((size_t)n * (pix ? 4 : 1), st);
-    cur.alloc(3 * n, st);
-    const long long np = std::max(3 * n, seg.planes_floats());
+    for (int k = 0; k < 2; ++k)
+        field[k].alloc(seg.planes_floats(), st);
     nd.alloc(seg.planes_floats(), st);
     aux.alloc(seg.planes_floats(), st);
-    tmp.alloc(np, st);  // the Poisson iterate's planes, then the interleaved accumulated field
+    tmp.alloc(seg.planes_floats(), st);
     seg.planar = 1;
     part.alloc(seg.nblk, st);
     ctl.alloc(1, st);
     seg.Js = js.p;
-    seg.cur_d = cur.p;
-    seg.best_d = best;
+    seg.field[0] = field[0].p;
+    seg.field[1] = field[1].p;
     seg.new_d = nd.p;
     seg.aux_d = aux.p;
     seg.tmp_d = tmp.p;
@@ -105,27 +105,35 @@ void CdmLevel::init(const void* const* It_, const void* const* Is_, const std::s
     c.speed = p.speed;
     c.smoothing = p.smoothing;
     c.max_iter = 200;
+    c.cur = c.from = c.best = 1;
     h_ctl = c;
     REGB_CK(cudaMemcpyAsync(ctl.p, &h_ctl, sizeof(CdmCtl), cudaMemcpyHostToDevice, st));
-    REGB_CK(cudaMemcpyAsync(cur.p, best, sizeof(float) * 3 * n, cudaMemcpyDeviceToDevice, st));  // cur_d(best_d)
+    REGB_CK(launch_planes_from_xyz(best, seg, field[1].p, st));  // cur_d(best_d)
     d_seg.alloc(1, st);
     REGB_CK(cudaMemcpyAsync(d_seg.p, &seg, sizeof(CdmSeg), cudaMemcpyHostToDevice, st));
     REGB_CK(cudaStreamSynchronize(st));  // h_ctl / seg are stack-staged: keep the copies ordered before reuse
 }
 
+void CdmLevel::best_field(float* xyz, cudaStream_t st) const
+{
+    REGB_CK(launch_xyz_from_planes(field[h_ctl.best].p, seg, xyz, st));
+}
+
 void launch_iteration(const CdmSegs& L, int pix, const std::string& gtypes, cudaStream_t st, bool first)
 {
     // compose and differentiate each modality in turn (reg/cdm.hpp:422-434); the
-    // last gradient launch also makes the loop decisions
+    // last gradient launch also makes the loop decisions.  The first modality was composed
+    // when the field was made (once more here for levels that share a first iteration's launch)
     for (int m = 0; m < (int)gtypes.size(); ++m) {
-        REGB_CK(launch_cdm_compose(L, pix, st, m));
+        if (m || first)
+            REGB_CK(launch_cdm_compose(L, pix, st, m));
         REGB_CK(launch_cdm_gradient(L, pix, gtypes[m], st, m));
     }
-    REGB_CK(launch_cdm_poisson(L, st));  // + best_d copy
+    REGB_CK(launch_cdm_poisson(L, st));
     if (first)
         REGB_CK(launch_cdm_theta(L, st));
     REGB_CK(launch_cdm_accumulate(L, st));
-    REGB_CK(launch_cdm_smooth(L, st));
+    REGB_CK(launch_cdm_smooth_compose(L, pix, st));
 }
 
 void accumulate_displacement_device(const float* dis, float* new_dis, const int* dim, cudaStream_t st)
@@ -141,13 +149,13 @@ void accumulate_displacement_device(const float* dis, float* new_dis, const int*
     DevBuf<float> out(3 * n, st);
     DevBuf<CdmCtl> ctl(1, st);
     DevBuf<CdmSeg> d_seg(1, st);
-    seg.cur_d = const_cast<float*>(dis);
+    seg.field[0] = const_cast<float*>(dis);
     seg.aux_d = new_dis;
     seg.tmp_d = out.p;
     seg.ctl = ctl.p;
     REGB_CK(cudaMemcpyAsync(ctl.p, &c, sizeof(c), cudaMemcpyHostToDevice, st));
     REGB_CK(cudaMemcpyAsync(d_seg.p, &seg, sizeof(seg), cudaMemcpyHostToDevice, st));
-    REGB_CK(launch_cdm_accumulate(CdmSegs{d_seg.p, &seg, 1, seg.nblk, seg.pnb}, st));
+    REGB_CK(launch_cdm_accumulate(CdmSegs{d_seg.p, &seg, 1, seg.nblk, seg.pnb, seg.tnb}, st));
     REGB_CK(cudaMemcpyAsync(new_dis, out.p, sizeof(float) * 3 * n, cudaMemcpyDeviceToDevice, st));
     REGB_CK(cudaStreamSynchronize(st));  // c and seg are stack-staged
 }
@@ -260,7 +268,7 @@ regb_status cdm_register_multi(const void* const* d_It, const void* const* d_Is,
             // launch; the loop decisions live on the device, so iterations launched after
             // the loop has ended are no-ops
             constexpr int kIters = 4;
-            const CdmSegs one{run.d_seg.p, &run.seg, 1, run.seg.nblk, run.seg.pnb};
+            const CdmSegs one{run.d_seg.p, &run.seg, 1, run.seg.nblk, run.seg.pnb, run.seg.tnb};
             GraphExec g;
             g.capture([&](cudaStream_t cs) {
                 for (int k = 0; k < kIters; ++k)
@@ -279,6 +287,7 @@ regb_status cdm_register_multi(const void* const* d_It, const void* const* d_Is,
                     break;
             }
         }
+        run.best_field(best, st);
         iters += run.h_ctl.iters_run;
         count_cdm_level(run.h_ctl.iters_run, (long long)n, pix ? 4 : 1);
         if (run.h_ctl.done == 2)

@@ -4,13 +4,16 @@
 // stride over its voxels.
 //
 // One iteration of a level (reg/cdm.hpp:418-470) is the launch sequence
-//   compose -> gradient (+ loop decisions in its last block) -> 12 Poisson sweeps
-//   (the first also saves/restores best_d) -> theta, on a level's first iteration only ->
-//   accumulate -> smooth
-// The reference's host-side decisions (cost bookkeeping, cdm_improved, the
-// smoothing schedule, best_d save/restore, theta, the iteration cap) run on the
-// device against CdmCtl, so a level runs without any host round trip; every
-// kernel of an iteration reads ctl->done and returns once a level has left its loop.
+//   gradient (+ loop decisions in its last block) -> 12 Poisson sweeps -> theta, on a
+//   level's first iteration only -> accumulate -> smooth and compose
+// with a compose launch of its own ahead of the first iteration, and one ahead of the
+// gradient of each further modality.  The reference's host-side decisions (cost
+// bookkeeping, cdm_improved, the smoothing schedule, best_d save/restore, theta, the
+// iteration cap) run on the device against CdmCtl, so a level runs without any host round
+// trip; every kernel of an iteration reads ctl->done and returns once a level has left its
+// loop.  best_d's save and restore move no data: the field has two buffers, and CdmCtl says
+// which one holds the best field and which the current one (128^3: the copies took up to 40
+// us of an iteration of 330).
 #include <algorithm>
 #include <atomic>
 #include <cfloat>
@@ -30,11 +33,11 @@ int cdm_blocks_for(long long nvox)
 }
 
 // The segment entry a block of a launch over nseg entries works on: the last one
-// whose blk0 <= blockIdx.x.  Every warp finds it on its own with one ballot per 32
+// whose first block <= blockIdx.x.  Every warp finds it on its own with one ballot per 32
 // entries (all lanes active: this runs first in each kernel); a launch of one entry
 // reads nothing to find it.
-// POISSON: by the Poisson launches' numbering (pblk0).
-template <bool POISSON = false>
+// FIRST: the numbering of the launch's grid.
+template <int CdmSeg::*FIRST>
 __device__ __forceinline__ int seg_of_block(const CdmSeg* __restrict__ segs, int nseg)
 {
     if (nseg <= 1)
@@ -43,7 +46,7 @@ __device__ __forceinline__ int seg_of_block(const CdmSeg* __restrict__ segs, int
     int k = 0;
     for (int base = 0; base < nseg; base += 32) {
         const int i = base + lane;
-        const unsigned m = __ballot_sync(0xffffffffu, i < nseg && (POISSON ? segs[i].pblk0 : segs[i].blk0) <= b);
+        const unsigned m = __ballot_sync(0xffffffffu, i < nseg && segs[i].*FIRST <= b);
         k += __popc(m);
         if (m != 0xffffffffu)
             break;
@@ -55,9 +58,9 @@ __device__ __forceinline__ int seg_of_block(const CdmSeg* __restrict__ segs, int
 // entry takes the other, which has no lookup in its code at all and the entry as a kernel
 // argument (`one`): a trip to memory less before its first load, 0.3 us of a launch.
 #define SEG_ARGS const CdmSeg *__restrict__ segs, int nseg, const __grid_constant__ CdmSeg one
-#define SEG_OF(poisson) (MULTI ? segs[seg_of_block<poisson>(segs, nseg)] : one)
+#define SEG_OF(blk0) (MULTI ? segs[seg_of_block<&CdmSeg::blk0>(segs, nseg)] : one)
 #define SEG_BEGIN                                                  \
-    const CdmSeg& S = SEG_OF(false);                               \
+    const CdmSeg& S = SEG_OF(blk0);                               \
     const int blk = (int)blockIdx.x - (MULTI ? S.blk0 : 0);        \
     if (blk >= S.nblk)                                             \
         return;                                                    \
@@ -66,66 +69,8 @@ __device__ __forceinline__ int seg_of_block(const CdmSeg* __restrict__ segs, int
     const long long stride = (long long)S.nblk * blockDim.x;       \
     const long long first = (long long)blk * blockDim.x + threadIdx.x;
 
-// ------------------------------------------------------------------ compose
-// compose_displacement (numerical/dif.hpp:90-107, 260-285): Js = Is[mod] where the
-// displacement is exactly zero, else the trilinear sample at x + d; failed
-// samples are 0.
-template <typename T, bool MULTI>
-__global__ void __launch_bounds__(kCdmThreads) cdm_compose_kernel(SEG_ARGS, int mod)
-{
-    SEG_BEGIN
-    if (S.ctl->done || mod >= max(S.nmod, 1))
-        return;
-    const T* __restrict__ Is = (const T*)S.Is[mod];
-    T* __restrict__ Js = (T*)S.Js;
-    const float* __restrict__ cd = S.cur_d;
-    if (S.ndim == 2) {
-        // the 2-D form: vector<2> field, bilinear sample at (x + dx, y + dy)
-        for (long long i = first; i < n; i += stride) {
-            const float dx = cd[3 * i], dy = cd[3 * i + 1];
-            T v;
-            if (dx == 0.0f && dy == 0.0f)
-                v = Is[i];
-            else {
-                const int x = (int)(i % D.w), y = (int)(i / D.w);
-                float px = (float)x, py = (float)y;
-                px += dx;
-                py += dy;
-                Cell2 c;
-                v = T(0);
-                if (bilinear_cell(D, px, py, c))
-                    v = assign_pix<T>(cell_sum2(Is, D, c));
-            }
-            Js[i] = v;
-        }
-        return;
-    }
-    for (long long i = first; i < n; i += stride) {
-        const float dx = cd[3 * i], dy = cd[3 * i + 1], dz = cd[3 * i + 2];
-        T v;
-        if (dx == 0.0f && dy == 0.0f && dz == 0.0f)
-            v = Is[i];
-        else {
-            int x, y, z;
-            unflat((int)i, D, x, y, z);
-            float px = (float)x, py = (float)y, pz = (float)z;
-            px += dx;
-            py += dy;
-            pz += dz;
-            Cell c;
-            v = T(0);
-            if (trilinear_cell(D, px, py, pz, c))
-                v = assign_pix<T>(cell_sum(Is, D, c));
-        }
-        Js[i] = v;
-    }
-}
-
-__device__ void control_block(const CdmSeg& S, int mod);
-__device__ __forceinline__ bool last_block_of_segment(const CdmSeg& S);
-
-// Where voxel i's x component sits in the update field (new_d, aux_d): component planes of
-// padded rows, or interleaved xyz; y and z follow at a stride of update_comp.
+// Where voxel i's x component sits in the fields (field, new_d, aux_d, tmp_d): component
+// planes of padded rows, or interleaved xyz; y and z follow at a stride of update_comp.
 __device__ __forceinline__ long long update_index(const CdmSeg& S, long long i)
 {
     if (!S.planar)
@@ -138,6 +83,102 @@ __device__ __forceinline__ long long update_index(const CdmSeg& S, long long r, 
     return S.planar ? r * S.ppitch + x : 3 * (r * S.w + x);
 }
 __device__ __forceinline__ long long update_comp(const CdmSeg& S) { return S.planar ? S.pplane : 1; }
+
+// Fields whose offsets in bytes fit 32 bits and whose coordinates are exact floats: the
+// sampling loops then need one add an address, and no conversion unit.
+__device__ __forceinline__ bool narrow(const CdmSeg& S)
+{
+    return S.pplane < (1LL << 30) && max(S.w, max(S.h, S.d)) < (1 << 22);
+}
+// The cell of a point inside such a field: f[axis] = its two corners' coordinates, the weights
+// as trilinear_cell forms them; returns its first corner's offset in rows of `pitch`.
+__device__ __forceinline__ unsigned narrow_cell(float x, float y, float z, unsigned pitch, unsigned h, float (&f)[3][2],
+                                                float (&r)[8])
+{
+    int ix, iy, iz;
+    f[0][0] = floor_pos(x, ix);
+    f[1][0] = floor_pos(y, iy);
+    f[2][0] = floor_pos(z, iz);
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+        f[k][1] = f[k][0] + 1.0f;
+    const float p0 = x - f[0][0], p1 = y - f[1][0], p2 = z - f[2][0];
+    const float n0 = 1.0f - p0, n1 = 1.0f - p1, n2 = 1.0f - p2;
+    const float n0n1 = n0 * n1, p0n1 = p0 * n1, n0p1 = n0 * p1, p0p1 = p0 * p1;
+    r[0] = n0n1 * n2;
+    r[1] = p0n1 * n2;
+    r[2] = n0p1 * n2;
+    r[3] = p0p1 * n2;
+    r[4] = n0n1 * p2;
+    r[5] = p0n1 * p2;
+    r[6] = n0p1 * p2;
+    r[7] = p0p1 * p2;
+    return ((unsigned)iz * h + (unsigned)iy) * pitch + (unsigned)ix;
+}
+
+// ------------------------------------------------------------------ compose
+// compose_displacement (numerical/dif.hpp:90-107, 260-285): Js = Is[mod] where the
+// displacement is exactly zero, else the trilinear sample at x + d; failed
+// samples are 0.  2-D: vector<2> field, bilinear sample at (x + dx, y + dy).
+template <typename T>
+__device__ __forceinline__ T compose_pixel(const T* __restrict__ Is, const Dim3& D, int ndim, int i, int x, int y, int z,
+                                           float dx, float dy, float dz)
+{
+    if (dx == 0.0f && dy == 0.0f && (ndim == 2 || dz == 0.0f))
+        return __ldg(Is + i);
+    const float px = (float)x + dx, py = (float)y + dy;
+    if (ndim == 2) {
+        Cell2 c;
+        return bilinear_cell(D, px, py, c) ? assign_pix<T>(cell_sum2(Is, D, c)) : T(0);
+    }
+    Cell c;
+    return trilinear_cell(D, px, py, (float)z + dz, c) ? assign_pix<T>(cell_sum(Is, D, c)) : T(0);
+}
+
+// The same in 3-D for a voxel of a narrow() level.
+__device__ __forceinline__ float pix_float(const uint8_t* p) { return u8_to_f(__ldg(p)); }
+__device__ __forceinline__ float pix_float(const float* p) { return __ldg(p); }
+template <typename T>
+__device__ __forceinline__ T compose_narrow(const T* __restrict__ Is, const SampleGeo& G, unsigned i, int x, int y, int z,
+                                            float dx, float dy, float dz)
+{
+    if (dx == 0.0f && dy == 0.0f && dz == 0.0f)
+        return __ldg(Is + i);
+    const float px = u8_to_f(x) + dx, py = u8_to_f(y) + dy, pz = u8_to_f(z) + dz;
+    if ((px < 0.0f || py < 0.0f || pz < 0.0f) || !(px < G.wl && py < G.hl && pz < G.dl))
+        return T(0);
+    float f[3][2], r[8], acc = 0.0f;
+    const unsigned b = narrow_cell(px, py, pz, (unsigned)G.w, (unsigned)G.h, f, r);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const unsigned off = (b + (k >> 1 & 1) * G.w + (k >> 2) * G.wh) * (unsigned)sizeof(T);
+        const float v = pix_float((const T*)((const char*)Is + off) + (k & 1));
+        acc = k ? acc + v * r[k] : v * r[k];
+    }
+    return assign_pix<T>(acc);
+}
+
+template <typename T, bool MULTI>
+__global__ void __launch_bounds__(kCdmThreads) cdm_compose_kernel(SEG_ARGS, int mod)
+{
+    SEG_BEGIN
+    if (S.ctl->done || mod >= max(S.nmod, 1))
+        return;
+    const T* __restrict__ Is = (const T*)S.Is[mod];
+    T* __restrict__ Js = (T*)S.Js;
+    const float* __restrict__ f = S.field[S.ctl->cur];
+    const long long cs = update_comp(S);
+    for (long long i = first; i < n; i += stride) {
+        const long long o = update_index(S, i);
+        const float dx = f[o], dy = f[o + cs], dz = f[o + 2 * cs];
+        int x, y, z;
+        unflat((int)i, D, x, y, z);
+        Js[i] = compose_pixel(Is, D, S.ndim, (int)i, x, y, z, dx, dy, dz);
+    }
+}
+
+__device__ void control_block(const CdmSeg& S, int mod);
+__device__ __forceinline__ bool last_block_of_segment(const CdmSeg& S);
 
 // ------------------------------------------------------------------ gradient
 // x / m rounded like the division, for the window sizes m <= 125 and r = RN(1 / m): the
@@ -434,7 +475,7 @@ template <bool MULTI>
 __global__ void __launch_bounds__(kUThreads) cdm_gradient_box_u8_kernel(SEG_ARGS,
                                                                          int mod)
 {
-    const CdmSeg& S = SEG_OF(false);
+    const CdmSeg& S = SEG_OF(blk0);
     const int blk = (int)blockIdx.x - (MULTI ? S.blk0 : 0);
     if (blk >= S.nblk)
         return;
@@ -615,7 +656,7 @@ template <bool MULTI>
 __global__ void __launch_bounds__(kFThreads, 3) cdm_gradient_r_f32_kernel(SEG_ARGS,
                                                                           int mod)
 {
-    const CdmSeg& S = SEG_OF(false);
+    const CdmSeg& S = SEG_OF(blk0);
     const int blk = (int)blockIdx.x - (MULTI ? S.blk0 : 0);
     if (blk >= S.nblk)
         return;
@@ -697,8 +738,6 @@ __device__ void control_step(CdmCtl* c, int nm, int mod, float mean_cost)
     c->mod_cost[mod] = mean_cost;
     if (mod + 1 < nm)
         return;
-    c->save_best = 0;
-    c->restore = 0;
     if (c->index >= c->max_iter) {
         c->done = 1;
         return;
@@ -718,7 +757,7 @@ __device__ void control_step(CdmCtl* c, int nm, int mod, float mean_cost)
     if (cur < c->best_cost) {
         c->best_cost = cur;
         if (c->index)
-            c->save_best = 1;
+            c->best = c->cur;
     }
     if (!cdm_improved_dev(c)) {
         if (c->cur_smoothing <= c->smoothing) {
@@ -726,10 +765,15 @@ __device__ void control_step(CdmCtl* c, int nm, int mod, float mean_cost)
             ++c->iters_run;
             return;
         }
-        c->restore = 1;
+        c->cur = c->best;
         c->cur_smoothing *= 0.5f;
         c->ncost = 0;
     }
+    // this iteration's field goes where the best one is not; without smoothing the field
+    // stays what it is
+    c->from = c->cur;
+    if (c->cur_smoothing != 0.0f)
+        c->cur = 1 - c->best;
     ++c->index;
     ++c->iters_run;
 }
@@ -795,6 +839,9 @@ __device__ __forceinline__ bool last_block_of_segment(const CdmSeg& S)
 constexpr int kPThreads = 256;
 constexpr int kPSweeps = 12;  // reg/cdm.hpp:165
 static_assert(kPSweeps % 2 == 0, "the result lands in aux_d");
+// The tail launches (accumulate, smooth and compose): a block takes kTile positions of one
+// plane, four a thread.
+constexpr int kTThreads = 128, kTile = 4 * kTThreads, kAVox = 2;
 
 // Launch shapes that follow from a level's dims alone.
 void cdm_set_dims(CdmSeg& s, int w, int h, int d)
@@ -819,6 +866,7 @@ void cdm_set_dims(CdmSeg& s, int w, int h, int d)
             break;
         }
     s.pnb = (int)(tiles * ((d + s.pdz - 1) / s.pdz));
+    s.tnb = (int)((s.ppitch * h + kTile - 1) / kTile * d);
 }
 
 // inv_d2 = -0.5 / dimension (reg/cdm.hpp:163,175): -1/6 in 3-D, -1/4 in 2-D.  A 2-D
@@ -835,6 +883,14 @@ __device__ __forceinline__ float4 load_now(const float4* __restrict__ p, bool ok
     float4 f = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     if (ok)
         asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(f.x), "=f"(f.y), "=f"(f.z), "=f"(f.w) : "l"(p));
+    return f;
+}
+
+__device__ __forceinline__ float load_now(const float* __restrict__ p, bool ok)
+{
+    float f = 0.0f;
+    if (ok)
+        asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(f) : "l"(p));
     return f;
 }
 
@@ -927,19 +983,16 @@ __device__ void poisson_flat(const CdmSeg& S, const float* __restrict__ in, cons
 }
 
 // One sweep.  FIRST: its input is new_d * (-1/6) formed on the fly (the same float product
-// the reference stores), its output tmp_d; it also applies this iteration's best_d save /
-// restore (reg/cdm.hpp:447-457), which the reference performs before its Poisson solve --
-// even on the iteration that leaves the loop.  Otherwise parity picks aux_d -> tmp_d or
+// the reference stores), its output tmp_d.  Otherwise parity picks aux_d -> tmp_d or
 // tmp_d -> aux_d (the last sweep).
 template <bool FIRST, bool MULTI>
 __global__ void __launch_bounds__(kPThreads, 4) cdm_poisson_kernel(SEG_ARGS, int parity)
 {
-    const CdmSeg& S = SEG_OF(true);
+    const CdmSeg& S = SEG_OF(pblk0);
     const int tile = (int)blockIdx.x - (MULTI ? S.pblk0 : 0);
     if (tile >= S.pnb)
         return;
-    const CdmCtl* c = S.ctl;
-    const int done = c->done;
+    const int done = S.ctl->done;
     // component slowest, then z chunks: the blocks in flight share planes
     const int per = S.pnb / 3, comp = tile / per, t = tile % per;
     const float* const rhs = S.new_d + comp * S.pplane;
@@ -960,21 +1013,6 @@ __global__ void __launch_bounds__(kPThreads, 4) cdm_poisson_kernel(SEG_ARGS, int
         else
             poisson_walk<FIRST, false>(S, in4, rhs4, out4, q, z0, z1, done);
     }
-    if (FIRST) {  // (last: the sweep reads neither field)
-        const long long n3 = 3LL * S.w * S.h * S.d;
-        const float* src = nullptr;
-        float* dst = nullptr;
-        if (c->save_best) {
-            src = S.cur_d;
-            dst = S.best_d;
-        } else if (c->restore) {
-            src = S.best_d;
-            dst = S.cur_d;
-        }
-        if (dst)
-            for (long long i = (long long)tile * kPThreads + threadIdx.x; i < n3; i += (long long)S.pnb * kPThreads)
-                dst[i] = src[i];
-    }
 }
 
 // An interleaved xyz field to the component planes of a segment's scratch, and back.
@@ -984,7 +1022,7 @@ __global__ void __launch_bounds__(kCdmThreads) planes_from_xyz_kernel(const floa
 {
     const long long n = D.n();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const long long r = i / D.w, o = r * pitch + (i - r * D.w);
+        const long long r = (unsigned)i / (unsigned)D.w, o = r * pitch + (i - r * D.w);
 #pragma unroll
         for (int c = 0; c < 3; ++c)
             planes[o + c * plane] = __ldg(xyz + 3 * i + c);
@@ -997,7 +1035,7 @@ __global__ void __launch_bounds__(kCdmThreads) xyz_from_planes_kernel(const floa
 {
     const long long n = D.n();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const long long r = i / D.w, o = r * pitch + (i - r * D.w);
+        const long long r = (unsigned)i / (unsigned)D.w, o = r * pitch + (i - r * D.w);
 #pragma unroll
         for (int c = 0; c < 3; ++c)
             xyz[3 * i + c] = __ldg(planes + o + c * plane);
@@ -1060,109 +1098,163 @@ __global__ void __launch_bounds__(kCdmThreads) cdm_theta_kernel(SEG_ARGS)
 // new_d *= speed/theta (reg/cdm.hpp:467) fused with accumulate_displacement
 // (numerical/dif.hpp:166-186): out = (cur_d + id)(x + new_d) - x where new_d is
 // non-zero and the sample lands inside, else cur_d.  The mapping cur_d + id is
-// formed per corner exactly as displacement_to_mapping stores it.
-template <bool MULTI>
-__global__ void __launch_bounds__(kCdmThreads) cdm_accumulate_kernel(SEG_ARGS)
+// formed per corner exactly as displacement_to_mapping stores it.  The 2-D form is the
+// bilinear sample of the mapping cur_d + (x, y); z stays 0.
+struct Accumulate {
+    const float *__restrict__ nd, *__restrict__ cd;
+    float* __restrict__ out;
+    Dim3 D;
+    int ndim;
+    float scale;
+};
+// One voxel whose x component sits at o; cs, sx, sy, sz: strides of a component, voxel, row
+// and plane.
+__device__ __forceinline__ void accumulate_voxel(const Accumulate& A, int x, int y, int z, long long o, long long cs, int sx,
+                                                 long long sy, long long sz, float dx, float dy, float dz)
 {
+    dx *= A.scale;
+    dy *= A.scale;
+    dz = A.ndim == 2 ? 0.0f : dz * A.scale;
+    bool ok = false;
+    float ax = 0.0f, ay = 0.0f, az = 0.0f;
+    if (dx != 0.0f || dy != 0.0f || dz != 0.0f) {
+        dx += (float)x;
+        dy += (float)y;
+        dz += (float)z;
+        const int bx = (int)dx, by = (int)dy, bz = (int)dz;
+        const float fx[2] = {(float)bx, (float)(bx + 1)}, fy[2] = {(float)by, (float)(by + 1)};
+        if (A.ndim == 2) {
+            Cell2 cl;
+            ok = bilinear_cell(A.D, dx, dy, cl);
+            if (ok) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const float* q = A.cd + (by + (k >> 1)) * sy + (long long)bx * sx + (k & 1) * sx;
+                    const float mx = q[0] + fx[k & 1], my = q[cs] + fy[k >> 1];
+                    ax = k ? ax + mx * cl.r[k] : mx * cl.r[k];
+                    ay = k ? ay + my * cl.r[k] : my * cl.r[k];
+                }
+            }
+        } else {
+            Cell cl;
+            ok = trilinear_cell(A.D, dx, dy, dz, cl);
+            if (ok) {
+                const float fz[2] = {(float)bz, (float)(bz + 1)};
+                const float* const p = A.cd + bz * sz + by * sy + (long long)bx * sx;
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    const float* q = p + (k >> 2) * sz + (k >> 1 & 1) * sy + (k & 1) * sx;
+                    const float mx = q[0] + fx[k & 1], my = q[cs] + fy[k >> 1 & 1], mz = q[2 * cs] + fz[k >> 2];
+                    ax = k ? ax + mx * cl.r[k] : mx * cl.r[k];
+                    ay = k ? ay + my * cl.r[k] : my * cl.r[k];
+                    az = k ? az + mz * cl.r[k] : mz * cl.r[k];
+                }
+            }
+        }
+    }
+    A.out[o] = ok ? ax - (float)x : A.cd[o];
+    A.out[o + cs] = ok ? ay - (float)y : A.cd[o + cs];
+    A.out[o + 2 * cs] = A.ndim == 2 ? 0.0f : ok ? az - (float)z : A.cd[o + 2 * cs];
+}
+
+// Interleaved fields (one accumulate_displacement).
+__global__ void __launch_bounds__(kCdmThreads) cdm_accumulate_xyz_kernel(SEG_ARGS)
+{
+    constexpr bool MULTI = false;
     SEG_BEGIN
     const CdmCtl* c = S.ctl;
     if (c->done)
         return;
-    const float scale = c->scale;
-    const float* __restrict__ nd = S.aux_d;
-    const long long cs = update_comp(S);
-    const float* __restrict__ cd = S.cur_d;
-    float* __restrict__ out = S.tmp_d;
-    const int w = D.w, wh = D.wh();
-    if (S.ndim == 2) {
-        // the 2-D form: bilinear sample of the mapping cur_d + (x, y); z stays 0
-        for (long long i = first; i < n; i += stride) {
-            const long long o = update_index(S, i);
-            float dx = nd[o] * scale, dy = nd[o + cs] * scale;
-            const int x = (int)(i % w), y = (int)(i / w);
-            bool ok = false;
-            if (dx != 0.0f || dy != 0.0f) {
-                dx += (float)x;
-                dy += (float)y;
-                Cell2 cl;
-                if (bilinear_cell(D, dx, dy, cl)) {
-                    const int b = cl.base, bx = b % w, by = b / w;
-                    const int off[4] = {0, 1, w, w + 1};
-                    const int ox[4] = {0, 1, 0, 1};
-                    const int oy[4] = {0, 0, 1, 1};
-                    float ax = 0.f, ay = 0.f;
+    const Accumulate A{S.aux_d, S.field[c->from], S.tmp_d, D, S.ndim, c->scale};
+    for (long long i = first; i < n; i += stride) {
+        int x, y, z;
+        unflat((int)i, D, x, y, z);
+        const long long o = 3 * i;
+        accumulate_voxel(A, x, y, z, o, 1, 3, 3LL * D.w, 3LL * D.wh(), A.nd[o], A.nd[o + 1], A.nd[o + 2]);
+    }
+}
+
+// Component planes: 24 gathers a voxel, whose lanes take neighbouring floats.  Bound by the
+// chain flag -> update -> cell -> gathers and the L2 traffic of the corner planes; a block
+// takes kTile positions of one plane, so that the last wave of a launch is short.
+// 91x109x91: 14.5 us on interleaved fields with a grid-wide stride, 11.7 so; with 1 / 4 voxels
+// a thread 14.9 / 12.4, 32^3 3.5 us against 2.8 / 6.0.
+constexpr int kAThreads = kTile / kAVox, kABlocks = 1280 / kAThreads;
+template <bool MULTI>
+__global__ void __launch_bounds__(kAThreads, kABlocks) cdm_accumulate_kernel(SEG_ARGS)
+{
+    const CdmSeg& S = SEG_OF(tblk0);
+    const int tile = (int)blockIdx.x - (MULTI ? S.tblk0 : 0);
+    if (tile >= S.tnb)
+        return;
+    const CdmCtl* c = S.ctl;
+    const Dim3 D{S.w, S.h, S.d};
+    const unsigned pitch = (unsigned)S.ppitch, plane = pitch * (unsigned)D.h;
+    const int tiles = S.tnb / D.d, z = tile / tiles;
+    const unsigned p0 = (unsigned)(tile - z * tiles) * kTile + threadIdx.x;
+    const long long cs = S.pplane, z0 = (long long)z * plane;
+    // the update's loads go out before the loop flag is waited for
+    float n0[kAVox], n1[kAVox], n2[kAVox];
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        const float* q = cd + 3LL * (b + off[k]);
-                        const float mx = q[0] + (float)(bx + ox[k]);
-                        const float my = q[1] + (float)(by + oy[k]);
-                        if (k == 0) {
-                            ax = mx * cl.r[0];
-                            ay = my * cl.r[0];
-                        } else {
-                            ax += mx * cl.r[k];
-                            ay += my * cl.r[k];
-                        }
-                    }
-                    out[3 * i] = ax - (float)x;
-                    out[3 * i + 1] = ay - (float)y;
-                    ok = true;
-                }
-            }
-            if (!ok) {
-                out[3 * i] = cd[3 * i];
-                out[3 * i + 1] = cd[3 * i + 1];
-            }
-            out[3 * i + 2] = 0.0f;
+    for (int k = 0; k < kAVox; ++k) {
+        const unsigned p = p0 + kAThreads * k;
+        const float* const q = S.aux_d + z0 + p;
+        n0[k] = load_now(q, p < plane);
+        n1[k] = load_now(q + cs, p < plane);
+        n2[k] = load_now(q + 2 * cs, p < plane);
+    }
+    const int done = c->done, from = c->from;
+    const float scale = c->scale;
+    if (done)
+        return;
+    const float* __restrict__ const cd = S.field[from];
+    if (S.ndim == 2 || !narrow(S)) {
+        const Accumulate A{S.aux_d, cd, S.tmp_d, D, S.ndim, scale};
+        for (unsigned p = p0; p < p0 - threadIdx.x + kTile; p += kAThreads) {
+            const int y = (int)(p / pitch), x = (int)(p - (unsigned)y * pitch);
+            const float* const q = A.nd + z0 + p;
+            if (p < plane && x < D.w)
+                accumulate_voxel(A, x, y, z, z0 + p, cs, 1, pitch, plane, q[0], q[cs], q[2 * cs]);
         }
         return;
     }
-    for (long long i = first; i < n; i += stride) {
-        const long long o = update_index(S, i);
-        float dx = nd[o] * scale, dy = nd[o + cs] * scale, dz = nd[o + 2 * cs] * scale;
-        int x, y, z;
-        unflat((int)i, D, x, y, z);
-        bool ok = false;
-        if (dx != 0.0f || dy != 0.0f || dz != 0.0f) {
-            dx += (float)x;
-            dy += (float)y;
-            dz += (float)z;
-            Cell cl;
-            if (trilinear_cell(D, dx, dy, dz, cl)) {
-                const int b = cl.base;
-                const int bx = b % w, by = (b / w) % D.h, bz = b / wh;
-                const int off[8] = {0, 1, w, w + 1, wh, wh + 1, wh + w, wh + w + 1};
-                const int ox[8] = {0, 1, 0, 1, 0, 1, 0, 1};
-                const int oy[8] = {0, 0, 1, 1, 0, 0, 1, 1};
-                const int oz[8] = {0, 0, 0, 0, 1, 1, 1, 1};
-                float ax = 0.f, ay = 0.f, az = 0.f;
+    // below, offsets in bytes fit 32 bits and coordinates are exact floats
+    const SampleGeo G{D.w, D.h, 0, (float)(D.w - 1), (float)(D.h - 1), (float)(D.d - 1)};
+    const char* const base[3] = {(const char*)cd, (const char*)(cd + cs), (const char*)(cd + 2 * cs)};
+    int y = (int)(p0 / pitch), x = (int)(p0 - (unsigned)y * pitch);
 #pragma unroll
-                for (int k = 0; k < 8; ++k) {
-                    const float* q = cd + 3LL * (b + off[k]);
-                    const float mx = q[0] + (float)(bx + ox[k]);
-                    const float my = q[1] + (float)(by + oy[k]);
-                    const float mz = q[2] + (float)(bz + oz[k]);
-                    if (k == 0) {
-                        ax = mx * cl.r[0];
-                        ay = my * cl.r[0];
-                        az = mz * cl.r[0];
-                    } else {
-                        ax += mx * cl.r[k];
-                        ay += my * cl.r[k];
-                        az += mz * cl.r[k];
+    for (int k = 0; k < kAVox; ++k) {
+        const unsigned p = p0 + kAThreads * k;
+        if (p < plane && x < D.w) {
+            const float dx = n0[k] * scale, dy = n1[k] * scale, dz = n2[k] * scale;
+            const float X = u8_to_f(x), Y = u8_to_f(y), Z = u8_to_f(z), px = dx + X, py = dy + Y, pz = dz + Z;
+            float* const o = S.tmp_d + z0 + p;
+            if (!(dx == 0.0f && dy == 0.0f && dz == 0.0f) && !(px < 0.0f || py < 0.0f || pz < 0.0f) && px < G.wl &&
+                py < G.hl && pz < G.dl) {
+                float f[3][2], r[8];
+                const unsigned b = 4u * narrow_cell(px, py, pz, pitch, (unsigned)D.h, f, r);
+                float a[3];
+#pragma unroll
+                for (int v = 0; v < 8; ++v) {
+                    const unsigned off = b + 4u * ((v >> 1 & 1) * pitch + (v >> 2) * plane);
+#pragma unroll
+                    for (int t = 0; t < 3; ++t) {
+                        const float m = __ldg((const float*)(base[t] + off) + (v & 1)) + f[t][v >> t & 1];
+                        a[t] = v ? a[t] + m * r[v] : m * r[v];
                     }
                 }
-                out[3 * i] = ax - (float)x;
-                out[3 * i + 1] = ay - (float)y;
-                out[3 * i + 2] = az - (float)z;
-                ok = true;
+                o[0] = a[0] - X;
+                o[cs] = a[1] - Y;
+                o[2 * cs] = a[2] - Z;
+            } else {
+                o[0] = __ldg(cd + z0 + p);
+                o[cs] = __ldg(cd + z0 + p + cs);
+                o[2 * cs] = __ldg(cd + z0 + p + 2 * cs);
             }
         }
-        if (!ok) {
-            out[3 * i] = cd[3 * i];
-            out[3 * i + 1] = cd[3 * i + 1];
-            out[3 * i + 2] = cd[3 * i + 2];
-        }
+        if (k + 1 < kAVox)
+            for (x += kAThreads; x >= (int)pitch; x -= (int)pitch)
+                ++y;
     }
 }
 
@@ -1170,9 +1262,15 @@ __global__ void __launch_bounds__(kCdmThreads) cdm_accumulate_kernel(SEG_ARGS)
 // cdm_smooth (reg/cdm.hpp:302-366): cur_d = d*(1-s) + (s/6) * (d[+1] + d[-1] +
 // d[+w] + d[-w] + d[+wh] + d[-wh]) by flat index; s == 0 leaves cur_d as it is.
 // 2-D: s/4 and four neighbours (the +-wh taps of a d == 1 level fall outside).
-template <bool MULTI>
+__device__ __forceinline__ float smooth_weight(const CdmSeg& S, float sm)
+{
+    return sm / (2.0f * (S.ndim == 2 ? 2.0f : 3.0f));  // smoothing / (2 * dimension)
+}
+
+// An interleaved field, a float a thread.
 __global__ void __launch_bounds__(kCdmThreads) cdm_smooth_kernel(SEG_ARGS)
 {
+    constexpr bool MULTI = false;
     SEG_BEGIN
     const CdmCtl* c = S.ctl;
     if (c->done)
@@ -1180,11 +1278,9 @@ __global__ void __launch_bounds__(kCdmThreads) cdm_smooth_kernel(SEG_ARGS)
     const float sm = c->cur_smoothing;
     if (sm == 0.0f)
         return;
-    const float w_6 = sm / (2.0f * (S.ndim == 2 ? 2.0f : 3.0f));  // smoothing / (2 * dimension)
-    const float w_1 = 1.0f - sm;
+    const float w_6 = smooth_weight(S, sm), w_1 = 1.0f - sm;
     const float* __restrict__ d = S.tmp_d;
-    float* __restrict__ dd = S.cur_d;
-    // one float of the interleaved array per thread (see the Poisson sweep)
+    float* __restrict__ dd = S.field[c->cur];
     const long long N3 = 3 * n, w3 = 3 * (long long)D.w, wh3 = 3 * (long long)D.wh();
     for (long long f = first; f < N3; f += stride) {
         float v = 0.0f;
@@ -1196,6 +1292,116 @@ __global__ void __launch_bounds__(kCdmThreads) cdm_smooth_kernel(SEG_ARGS)
         if (f >= wh3) v += d[f - wh3];
         v *= w_6;
         dd[f] = d[f] * w_1 + v;
+    }
+}
+
+// An iteration's smoothing and the next one's compose of the first modality in one pass over
+// the component planes: a thread smooths a float4 of each component (taps as in the Poisson
+// sweeps), and a warp hands its 128 voxels over through shared memory to sample them 32
+// neighbours at a time.  91x109x91 uint8: 17.9 us as two launches over interleaved fields
+// (seven scalar loads a float), 11.8 so.
+template <typename T, bool MULTI>
+__global__ void __launch_bounds__(kTThreads) cdm_smooth_compose_kernel(SEG_ARGS)
+{
+    const CdmSeg& S = SEG_OF(tblk0);
+    const int tile = (int)blockIdx.x - (MULTI ? S.tblk0 : 0);
+    if (tile >= S.tnb)
+        return;
+    const CdmCtl* c = S.ctl;
+    if (c->done)
+        return;
+    const float sm = c->cur_smoothing;
+    const float w_6 = smooth_weight(S, sm), w_1 = 1.0f - sm;
+    float* const dst = S.field[c->cur];
+    const T* __restrict__ const Is = (const T*)S.Is[0];
+    T* __restrict__ const Js = (T*)S.Js;
+    const Dim3 D{S.w, S.h, S.d};
+    const unsigned pitch = (unsigned)S.ppitch;
+    const int tiles = S.tnb / D.d, z = tile / tiles, tp = (tile - z * tiles) * kTile;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x & ~31;
+    __shared__ float4 field[3][kTThreads];
+    if ((pitch & 3) == 0) {
+        const unsigned P = pitch / 4, plane = P * (unsigned)D.h, total = plane * (unsigned)D.d;
+        const unsigned q = (unsigned)tp / 4 + threadIdx.x, xq = q % P, i = (unsigned)z * plane + q;
+        const int rem = D.w & 3;
+        const bool on = q < plane, row_end = xq == P - 1;
+        const bool fix1 = row_end && rem == 1, fix2 = row_end && rem == 2, fix3 = row_end && rem == 3;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const float4* const in = reinterpret_cast<const float4*>(S.tmp_d + k * S.pplane);
+            float4* const out = reinterpret_cast<float4*>(dst + k * S.pplane);
+            auto at = [&](unsigned j) {
+                return on && j < total ? __ldg(in + j) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            };
+            auto one = [&](long long j) {
+                return on && j >= 0 && j < 4LL * total ? __ldg(reinterpret_cast<const float*>(in) + j) : 0.0f;
+            };
+            float4 r;
+            if (sm == 0.0f)
+                r = on ? out[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            else {
+                const float4 cur = at(i), ya = at(i - P), yb = at(i + P), down = at(i - plane), up = at(i + plane);
+                const float tail = fix1 ? cur.x : fix2 ? cur.y : fix3 ? cur.z : cur.w;
+                float xl = __shfl_up_sync(0xffffffffu, tail, 1), xr = __shfl_down_sync(0xffffffffu, cur.x, 1);
+                if (lane == 0)
+                    xl = one(4LL * i - 1 - (xq == 0 && rem ? 4 - rem : 0));
+                if (lane == 31 || q + 1 == plane)
+                    xr = one(4LL * i + 4);
+                const float n1 = fix1 ? xr : cur.y, n2 = fix2 ? xr : cur.z, n3 = fix3 ? xr : cur.w;
+                r.x = cur.x * w_1 + ((((((0.0f + n1) + xl) + yb.x) + ya.x) + up.x) + down.x) * w_6;
+                r.y = cur.y * w_1 + ((((((0.0f + n2) + cur.x) + yb.y) + ya.y) + up.y) + down.y) * w_6;
+                r.z = cur.z * w_1 + ((((((0.0f + n3) + cur.y) + yb.z) + ya.z) + up.z) + down.z) * w_6;
+                r.w = cur.w * w_1 + ((((((0.0f + xr) + cur.z) + yb.w) + ya.w) + up.w) + down.w) * w_6;
+                if (on)
+                    out[i] = r;
+            }
+            field[k][threadIdx.x] = r;
+        }
+    } else {  // unpadded rows: a float at a time
+        const long long w = D.w, wh = D.wh(), n = D.n();
+        for (int k = 0; k < 3; ++k)
+            for (int j = 0; j < 4; ++j) {
+                const int p = tp + 4 * warp + 32 * j + lane;
+                const long long i = z * wh + p;
+                const float* __restrict__ const d = S.tmp_d + k * S.pplane;
+                float* const out = dst + k * S.pplane;
+                if (p >= wh)
+                    continue;
+                float r;
+                if (sm == 0.0f)
+                    r = out[i];
+                else {
+                    float v = 0.0f;
+                    if (i + 1 < n) v += d[i + 1];
+                    if (i >= 1) v += d[i - 1];
+                    if (i + w < n) v += d[i + w];
+                    if (i >= w) v += d[i - w];
+                    if (i + wh < n) v += d[i + wh];
+                    if (i >= wh) v += d[i - wh];
+                    v *= w_6;
+                    r = d[i] * w_1 + v;
+                    out[i] = r;
+                }
+                reinterpret_cast<float*>(field[k])[p - tp] = r;
+            }
+    }
+    __syncwarp();
+    const bool fast = S.ndim != 2 && narrow(S);
+    const SampleGeo G = sample_geo(D);
+    const int v0 = 4 * warp + lane;
+    int y = (int)((unsigned)(tp + v0) / pitch), x = (int)((unsigned)(tp + v0) - (unsigned)y * pitch);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int v = v0 + 32 * k;
+        const float dx = reinterpret_cast<const float*>(field[0])[v], dy = reinterpret_cast<const float*>(field[1])[v],
+                    dz = reinterpret_cast<const float*>(field[2])[v];
+        if (y < D.h && x < D.w) {
+            const int j = (z * D.h + y) * D.w + x;
+            Js[j] = fast ? compose_narrow(Is, G, (unsigned)j, x, y, z, dx, dy, dz)
+                         : compose_pixel(Is, D, S.ndim, j, x, y, z, dx, dy, dz);
+        }
+        for (x += 32; x >= (int)pitch; x -= (int)pitch)
+            ++y;
     }
 }
 
@@ -1461,14 +1667,31 @@ cudaError_t launch_cdm_theta(const CdmSegs& L, cudaStream_t st)
 
 cudaError_t launch_cdm_accumulate(const CdmSegs& L, cudaStream_t st)
 {
-    SEG_LAUNCH(cdm_accumulate_kernel<true>, cdm_accumulate_kernel<false>, kCdmThreads, 0);
+    if (L.host->planar) {
+        auto kernel = L.n > 1 ? cdm_accumulate_kernel<true> : cdm_accumulate_kernel<false>;
+        kernel<<<L.tblocks, kAThreads, 0, st>>>(L.dev, L.n, *L.host);
+    } else if (L.n == 1)
+        cdm_accumulate_xyz_kernel<<<L.blocks, kCdmThreads, 0, st>>>(L.dev, L.n, *L.host);
+    else
+        return cudaErrorInvalidValue;
     count_launch();
     return cudaGetLastError();
 }
 
 cudaError_t launch_cdm_smooth(const CdmSegs& L, cudaStream_t st)
 {
-    SEG_LAUNCH(cdm_smooth_kernel<true>, cdm_smooth_kernel<false>, kCdmThreads, 0);
+    if (L.n != 1 || L.host->planar)
+        return cudaErrorInvalidValue;
+    cdm_smooth_kernel<<<L.blocks, kCdmThreads, 0, st>>>(L.dev, L.n, *L.host);
+    count_launch();
+    return cudaGetLastError();
+}
+
+cudaError_t launch_cdm_smooth_compose(const CdmSegs& L, int pix, cudaStream_t st)
+{
+    auto kernel = L.n > 1 ? (pix ? cdm_smooth_compose_kernel<float, true> : cdm_smooth_compose_kernel<uint8_t, true>)
+                          : (pix ? cdm_smooth_compose_kernel<float, false> : cdm_smooth_compose_kernel<uint8_t, false>);
+    kernel<<<L.tblocks, kTThreads, 0, st>>>(L.dev, L.n, *L.host);
     count_launch();
     return cudaGetLastError();
 }

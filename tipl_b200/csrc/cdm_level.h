@@ -25,15 +25,17 @@ struct CdmLevel {
     CdmSeg seg{};
     CdmCtl h_ctl{};
     DevBuf<uint8_t> js;
-    DevBuf<float> cur, nd, aux, tmp;
+    DevBuf<float> field[2], nd, aux, tmp;
     DevBuf<double> part;
     DevBuf<CdmCtl> ctl;
     DevBuf<CdmSeg> d_seg;
-    // It / Is: gtypes.size() modality pairs of one shape.  best is the level's in/out
-    // field (starts as the upsampled coarser result).
+    // It / Is: gtypes.size() modality pairs of one shape.  best is the field the level starts
+    // from (the upsampled coarser result).
     // ndim 2: a level of a 2-D registration (d == 1).
     void init(const void* const* It, const void* const* Is, const std::string& gtypes, int w, int h, int d, int pix,
-              const regb_cdm_param& p, float* best, cudaStream_t st, int ndim = 3);
+              const regb_cdm_param& p, const float* best, cudaStream_t st, int ndim = 3);
+    // The best field as of h_ctl, interleaved.
+    void best_field(float* xyz, cudaStream_t st) const;
 };
 
 // One iteration of every segment of L (reg/cdm.hpp:418-470); they share pix and the gradient

@@ -62,8 +62,9 @@ struct CdmCtl {
     int index;             // iteration of this level
     int max_iter;          // 200
     int done;              // 1 = loop left (break / iteration cap / theta 0), 2 = zero cost (failure)
-    int save_best;         // this iteration: best_d <- cur_d
-    int restore;           // this iteration: cur_d <- best_d
+    // which of the segment's two field buffers holds the current field (compose reads it, the
+    // smoothing writes it), the one this iteration starts from (accumulate reads it), the best
+    int cur, from, best;
     unsigned int theta_bits;  // max |new_d| of the first iteration (float bits)
     unsigned int ticket;
     float last_cost;
@@ -83,11 +84,10 @@ struct CdmSeg {
     const void* It[kCdmMaxModalities];  // template (fixed) image of each modality at this level
     const void* Is[kCdmMaxModalities];  // subject (moving) image of each modality at this level
     void* Js;         // composed subject (scratch, pixel type)
-    float* cur_d;     // current field
-    float* best_d;    // best field
+    float* field[2];  // the field's buffers (CdmCtl::cur, from, best)
     float* new_d;     // gradient (scratch)
     float* aux_d;     // Poisson iterate A / Poisson result (scratch)
-    float* tmp_d;     // Poisson iterate B / accumulated field, interleaved (scratch)
+    float* tmp_d;     // Poisson iterate B / accumulated field (scratch)
     double* cost_part;  // per-block partial cost sums (nblk entries)
     CdmCtl* ctl;
     // A launch over several segments (their entries back to back) has sum(nblk) blocks:
@@ -97,20 +97,21 @@ struct CdmSeg {
     // The Poisson launches' own grid: pnb blocks, pdz planes a thread; pblk0 numbers them as
     // blk0 does.
     int pblk0, pnb, pdz;
-    // planar: the update field (new_d, aux_d and the Poisson iterates in tmp_d) is held as
-    // component planes of pplane floats, rows ppitch apart, as the Poisson launches take
-    // it; else interleaved xyz
+    // and the grid of an iteration's last two launches (accumulate, smooth and compose)
+    int tblk0, tnb;
+    // planar: the fields (field, new_d, aux_d, tmp_d) are held as component planes of pplane
+    // floats, rows ppitch apart, as the Poisson launches take them; else interleaved xyz
     int planar;
     long long ppitch, pplane;
     long long planes_floats() const { return 3 * pplane; }
 };
 // The segments of one launch: n entries on the device and on the host (one entry alone is
-// passed to the kernels by value); blocks / pblocks: sum(nblk) / sum(pnb) over the entries,
-// whose blk0 / pblk0 number them.
+// passed to the kernels by value); blocks / pblocks / tblocks: sum(nblk) / sum(pnb) / sum(tnb)
+// over the entries, whose blk0 / pblk0 / tblk0 number them.
 struct CdmSegs {
     const CdmSeg* dev;
     const CdmSeg* host;
-    int n, blocks, pblocks;
+    int n, blocks, pblocks, tblocks;
 };
 // Sets a segment's dims and the launch shapes that follow from them.
 void cdm_set_dims(CdmSeg& s, int w, int h, int d);
@@ -151,11 +152,14 @@ cudaError_t launch_fixed_stats(const uint8_t* f, long long n, int32_t* hist, uns
 cudaError_t launch_cdm_compose(const CdmSegs& L, int pix, cudaStream_t st, int mod = 0);
 cudaError_t launch_cdm_gradient(const CdmSegs& L, int pix, int gradient_type,
                                 cudaStream_t st, int mod = 0);
-// 12 sweeps of planar segments; the first launch also applies best_d save/restore.
+// 12 sweeps of planar segments.
 cudaError_t launch_cdm_poisson(const CdmSegs& L, cudaStream_t st);
 cudaError_t launch_cdm_theta(const CdmSegs& L, cudaStream_t st);
 cudaError_t launch_cdm_accumulate(const CdmSegs& L, cudaStream_t st);
+// One interleaved segment.
 cudaError_t launch_cdm_smooth(const CdmSegs& L, cudaStream_t st);
+// The smoothing of planar segments and the next iteration's compose of Is[0].
+cudaError_t launch_cdm_smooth_compose(const CdmSegs& L, int pix, cudaStream_t st);
 
 // An interleaved field to the component planes of s and back.
 cudaError_t launch_planes_from_xyz(const float* xyz, const CdmSeg& s, float* planes, cudaStream_t st);

@@ -86,23 +86,25 @@ void CdmScheduler::loop()
             // one launch per group over exactly its blocks: each entry's blk0 counts the
             // blocks of the group's entries before it
             struct Group {
-                int g0, g1, blocks, pblocks;
+                int g0, g1, blocks, pblocks, tblocks;
                 bool first;
             };
             std::vector<Group> groups;
             for (int g0 = 0; g0 < n;) {
-                int g1 = g0, blocks = 0, pblocks = 0;
+                int g1 = g0, blocks = 0, pblocks = 0, tblocks = 0;
                 bool first = false;
                 while (g1 < n && key(order[g1]) == key(order[g0])) {
                     h_segs_.p[g1].blk0 = blocks;
                     h_segs_.p[g1].pblk0 = pblocks;
+                    h_segs_.p[g1].tblk0 = tblocks;
                     blocks += h_segs_.p[g1].nblk;
                     pblocks += h_segs_.p[g1].pnb;
+                    tblocks += h_segs_.p[g1].tnb;
                     first = first || !cur[order[g1]]->started;
                     cur[order[g1]]->started = true;
                     ++g1;
                 }
-                groups.push_back({g0, g1, blocks, pblocks, first});
+                groups.push_back({g0, g1, blocks, pblocks, tblocks, first});
                 g0 = g1;
             }
             REGB_CK(cudaEventRecord(ev_[0], st_));
@@ -110,7 +112,7 @@ void CdmScheduler::loop()
             for (int it = 0; it < iters_; ++it)
                 for (const Group& g : groups) {
                     const Entry* e = cur[order[g.g0]];
-                    launch_iteration(CdmSegs{segs_.p + g.g0, h_segs_.p + g.g0, g.g1 - g.g0, g.blocks, g.pblocks},
+                    launch_iteration(CdmSegs{segs_.p + g.g0, h_segs_.p + g.g0, g.g1 - g.g0, g.blocks, g.pblocks, g.tblocks},
                                      e->lvl->pix, e->lvl->gtypes, st_, it == 0 && g.first);
                 }
             REGB_CK(launch_cdm_status(segs_.p, n, status_.p, st_));
