@@ -1015,6 +1015,207 @@ __global__ void __launch_bounds__(kPThreads, 4) cdm_poisson_kernel(SEG_ARGS, int
     }
 }
 
+// ---- the 12 sweeps of a small level in one launch ----
+// A cluster of kPCluster blocks holds one component in shared memory: a block owns K planes and
+// a halo plane on either side, a thread a float4 column of them with its right-hand side in
+// registers.  A sweep reads one copy of the planes and writes the other; the outer planes also
+// go to the neighbouring blocks' halos over distributed shared memory, and a cluster barrier
+// ends it.  Taps, padding and arithmetic are poisson_walk's; a halo outside the field stays
+// zero.
+//
+// Bound by the barrier and the exchange (0.65 us a sweep at 16^3) on the smallest, then by issue.  Twelve launches of a sweep before, one so: 23x28x23 25 / 8.8
+// us, 32^3 24.6 / 10.8, 46x55x46 40 / 19, 64^3 40 / 32, and the gaps between the launches.
+// Larger levels do not fit: a plane has to be a block's columns, 16 blocks hold 64 planes.
+constexpr int kPCluster = 16, kPClusterThreads = 1024, kPClusterPlanes = 4;
+
+__device__ __forceinline__ void cluster_barrier()
+{
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// The address of p (shared memory of this block) in block `rank` of the cluster, and a store there.
+__device__ __forceinline__ unsigned remote_address(const float4* p, int rank)
+{
+    unsigned r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void store_remote(unsigned address, float4 v)
+{
+    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(address), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
+                 : "memory");
+}
+
+// The sweeps of a block with NZ planes from z0 on.  K: the planes of a full block, which place
+// the upper halo of the block below.  PAD: rows end within a float4.
+template <int NZ, bool PAD>
+__device__ __forceinline__ void poisson_block(const CdmSeg& S, float4* planes, int K, int rank, int comp)
+{
+    const unsigned P = (unsigned)(S.ppitch / 4), plane = P * (unsigned)S.h, copy = (K + 2) * plane;
+    const float c6 = poisson_weight(S);
+    const int z0 = rank * K, rem = S.w & 3, lane = threadIdx.x & 31;
+    // threads past the plane go through the last column's motions and store nothing
+    const unsigned q = min(threadIdx.x, plane - 1), xq = q % P;
+    const bool on = threadIdx.x < plane, row_end = PAD && xq == P - 1, first = lane == 0, last = lane == 31 || q + 1 == plane;
+    const bool fix1 = row_end && rem == 1, fix2 = row_end && rem == 2, fix3 = row_end && rem == 3;
+    const int left = -1 - (PAD && xq == 0 ? 4 - rem : 0);
+    const bool push_low = on && rank > 0, push_high = on && z0 + NZ < S.d;
+    const unsigned low = remote_address(planes + (K + 1) * plane + q, max(rank - 1, 0)),
+                   high = remote_address(planes + q, rank + (z0 + NZ < S.d ? 1 : 0));
+    const float4* const rhs = reinterpret_cast<const float4*>(S.new_d + comp * S.pplane) + (unsigned)z0 * plane + q;
+    float4* const out = reinterpret_cast<float4*>(S.aux_d + comp * S.pplane) + (unsigned)z0 * plane + q;
+    const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    auto scaled = [&](float4 f) { return make_float4(f.x * c6, f.y * c6, f.z * c6, f.w * c6); };
+    float4 b[NZ], v[NZ];
+#pragma unroll
+    for (int k = 0; k < NZ; ++k)
+        b[k] = __ldg(rhs + k * plane);
+    const float4 below = rank > 0 ? scaled(__ldg(rhs - plane)) : zero;
+    const float4 above = z0 + NZ < S.d ? scaled(__ldg(rhs + NZ * plane)) : zero;
+#pragma unroll
+    for (int k = 0; k < NZ; ++k)
+        v[k] = scaled(b[k]);
+    if (on) {  // the second copy's halos outside the field stay zero
+        planes[q] = below;
+        planes[(NZ + 1) * plane + q] = above;
+        planes[copy + q] = zero;
+        planes[copy + (NZ + 1) * plane + q] = zero;
+#pragma unroll
+        for (int k = 0; k < NZ; ++k)
+            planes[(k + 1) * plane + q] = v[k];
+    }
+    cluster_barrier();
+    auto sweep = [&](unsigned from, unsigned to, bool end) {
+        const float4* p = planes + from + plane + q;
+        float4* t = planes + to + plane + q;
+        float4 down = *(p - plane);
+        const float4 top = *(p + NZ * plane);
+#pragma unroll
+        for (int k = 0; k < NZ; ++k) {
+            const float4 cur = v[k], ya = *(p - P), yb = *(p + P), up = k + 1 < NZ ? v[k + 1 < NZ ? k + 1 : k] : top;
+            const float tail = fix1 ? cur.x : fix2 ? cur.y : fix3 ? cur.z : cur.w;
+            float xl = __shfl_up_sync(0xffffffffu, tail, 1), xr = __shfl_down_sync(0xffffffffu, cur.x, 1);
+            if (first)
+                xl = *(reinterpret_cast<const float*>(p) + left);
+            if (last)
+                xr = *(reinterpret_cast<const float*>(p) + 4);
+            const float n1 = fix1 ? xr : cur.y, n2 = fix2 ? xr : cur.z, n3 = fix3 ? xr : cur.w;
+            float4 n;
+            n.x = ((((((b[k].x - xl) - n1) - ya.x) - yb.x) - down.x) - up.x) * c6;
+            n.y = ((((((b[k].y - cur.x) - n2) - ya.y) - yb.y) - down.y) - up.y) * c6;
+            n.z = ((((((b[k].z - cur.y) - n3) - ya.z) - yb.z) - down.z) - up.z) * c6;
+            n.w = ((((((b[k].w - cur.z) - xr) - ya.w) - yb.w) - down.w) - up.w) * c6;
+            down = cur;
+            v[k] = n;
+            if (end) {
+                if (on)
+                    out[k * plane] = n;
+            } else {
+                if (on)
+                    *t = n;
+                if (k == 0 && push_low)
+                    store_remote(low + 16 * to, n);
+                if (k + 1 == NZ && push_high)
+                    store_remote(high + 16 * to, n);
+            }
+            p += plane;
+            t += plane;
+        }
+    };
+#pragma unroll 1
+    for (int k = 0; k + 1 < kPSweeps; ++k) {
+        sweep(k & 1 ? copy : 0, k & 1 ? 0 : copy, false);
+        cluster_barrier();
+    }
+    sweep(kPSweeps & 1 ? 0 : copy, 0, true);
+}
+
+template <int K, bool PAD>
+__global__ void __launch_bounds__(kPClusterThreads) cdm_poisson_cluster_kernel(const __grid_constant__ CdmSeg S)
+{
+    extern __shared__ float4 planes[];  // two copies of K + 2 planes
+    if (S.ctl->done)
+        return;
+    const int rank = (int)blockIdx.x % kPCluster, comp = (int)blockIdx.x / kPCluster;
+    const int nz = max(0, min(K, S.d - rank * K));  // the same for every thread of the block
+    if (nz == K)
+        poisson_block<K, PAD>(S, planes, K, rank, comp);
+    else if (K > 3 && nz == 3)
+        poisson_block<3, PAD>(S, planes, K, rank, comp);
+    else if (K > 2 && nz == 2)
+        poisson_block<2, PAD>(S, planes, K, rank, comp);
+    else if (K > 1 && nz == 1)
+        poisson_block<1, PAD>(S, planes, K, rank, comp);
+    else
+        for (int k = 0; k < kPSweeps; ++k)
+            cluster_barrier();
+}
+
+// The launch for a level of d <= K * kPCluster planes; cudaErrorNotSupported where the device
+// cannot hold a whole cluster.
+template <int K, bool PAD>
+cudaError_t launch_poisson_cluster(const CdmSeg& s, cudaStream_t st)
+{
+    auto config = [&](unsigned cols, cudaLaunchAttribute& attr) {
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = kPCluster;
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(3 * kPCluster);
+        cfg.blockDim = dim3((cols + 31) / 32 * 32);
+        cfg.dynamicSmemBytes = 2 * (K + 2) * cols * sizeof(float4);
+        cfg.stream = st;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        return cfg;
+    };
+    cudaLaunchAttribute attr{};
+    static std::atomic<unsigned long long> asked{0}, fits{0};
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess)
+        return e;
+    const unsigned long long bit = 1ull << (dev & 63);
+    if (!(asked.load() & bit)) {
+        e = cudaFuncSetAttribute(cdm_poisson_cluster_kernel<K, PAD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 2 * (K + 2) * kPClusterThreads * (int)sizeof(float4));
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(cdm_poisson_cluster_kernel<K, PAD>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        int clusters = 0;
+        if (e == cudaSuccess) {
+            const cudaLaunchConfig_t cfg = config(kPClusterThreads, attr);
+            e = cudaOccupancyMaxActiveClusters(&clusters, cdm_poisson_cluster_kernel<K, PAD>, &cfg);
+        }
+        if (e != cudaSuccess)
+            return e;
+        if (clusters > 0)
+            fits.fetch_or(bit);
+        asked.fetch_or(bit);
+    }
+    if (!(fits.load() & bit))
+        return cudaErrorNotSupported;
+    const cudaLaunchConfig_t cfg = config((unsigned)(s.ppitch / 4 * s.h), attr);
+    e = cudaLaunchKernelEx(&cfg, cdm_poisson_cluster_kernel<K, PAD>, s);
+    if (e == cudaSuccess)
+        count_launch();
+    return e;
+}
+
+// The sweeps of one level in clusters where it fits them, else cudaErrorNotSupported.
+cudaError_t launch_poisson_clusters(const CdmSeg& s, cudaStream_t st)
+{
+    if (s.ppitch % 4 || s.ppitch / 4 * s.h > kPClusterThreads)
+        return cudaErrorNotSupported;
+    static_assert(kPClusterPlanes == 4, "one instantiation for each number of planes");
+    switch ((s.d + kPCluster - 1) / kPCluster) {
+    case 1: return s.w & 3 ? launch_poisson_cluster<1, true>(s, st) : launch_poisson_cluster<1, false>(s, st);
+    case 2: return s.w & 3 ? launch_poisson_cluster<2, true>(s, st) : launch_poisson_cluster<2, false>(s, st);
+    case 3: return s.w & 3 ? launch_poisson_cluster<3, true>(s, st) : launch_poisson_cluster<3, false>(s, st);
+    case 4: return s.w & 3 ? launch_poisson_cluster<4, true>(s, st) : launch_poisson_cluster<4, false>(s, st);
+    default: return cudaErrorNotSupported;
+    }
+}
+
 // An interleaved xyz field to the component planes of a segment's scratch, and back.
 __global__ void __launch_bounds__(kCdmThreads) planes_from_xyz_kernel(const float* __restrict__ xyz, Dim3 D,
                                                                       long long pitch, long long plane,
@@ -1649,6 +1850,11 @@ cudaError_t launch_cdm_gradient(const CdmSegs& L, int pix, int gradient_type,
 
 cudaError_t launch_cdm_poisson(const CdmSegs& L, cudaStream_t st)
 {
+    if (L.n == 1) {
+        const cudaError_t e = launch_poisson_clusters(*L.host, st);
+        if (e != cudaErrorNotSupported)
+            return e;
+    }
     for (int k = 0; k < kPSweeps; ++k) {
         auto kernel = L.n > 1 ? (k ? cdm_poisson_kernel<false, true> : cdm_poisson_kernel<true, true>)
                               : (k ? cdm_poisson_kernel<false, false> : cdm_poisson_kernel<true, false>);
