@@ -120,7 +120,7 @@ struct OneSeg {
         std::memset(&c, 0, sizeof(c));
         c.max_iter = 200;
     }
-    CdmSegs segs() const { return CdmSegs{seg.p, &h, 1, h.nblk, h.pnb, h.tnb}; }
+    CdmSegs segs() const { return CdmSegs{seg.p, &h, 1, h.nblk, h.pnb, h.tnb, cdm_poisson_small(h)}; }
     void upload(cudaStream_t st)
     {
         REGB_CK(cudaMemcpyAsync(ctl.p, &c, sizeof(c), cudaMemcpyHostToDevice, st));

@@ -155,7 +155,7 @@ void accumulate_displacement_device(const float* dis, float* new_dis, const int*
     seg.ctl = ctl.p;
     REGB_CK(cudaMemcpyAsync(ctl.p, &c, sizeof(c), cudaMemcpyHostToDevice, st));
     REGB_CK(cudaMemcpyAsync(d_seg.p, &seg, sizeof(seg), cudaMemcpyHostToDevice, st));
-    REGB_CK(launch_cdm_accumulate(CdmSegs{d_seg.p, &seg, 1, seg.nblk, seg.pnb, seg.tnb}, st));
+    REGB_CK(launch_cdm_accumulate(CdmSegs{d_seg.p, &seg, 1, seg.nblk, seg.pnb, seg.tnb, 0}, st));
     REGB_CK(cudaMemcpyAsync(new_dis, out.p, sizeof(float) * 3 * n, cudaMemcpyDeviceToDevice, st));
     REGB_CK(cudaStreamSynchronize(st));  // c and seg are stack-staged
 }
@@ -268,7 +268,8 @@ regb_status cdm_register_multi(const void* const* d_It, const void* const* d_Is,
             // launch; the loop decisions live on the device, so iterations launched after
             // the loop has ended are no-ops
             constexpr int kIters = 4;
-            const CdmSegs one{run.d_seg.p, &run.seg, 1, run.seg.nblk, run.seg.pnb, run.seg.tnb};
+            const CdmSegs one{run.d_seg.p, &run.seg, 1, run.seg.nblk, run.seg.pnb, run.seg.tnb,
+                              cdm_poisson_small(run.seg)};
             GraphExec g;
             g.capture([&](cudaStream_t cs) {
                 for (int k = 0; k < kIters; ++k)

@@ -1058,7 +1058,7 @@ __device__ __forceinline__ void poisson_block(const CdmSeg& S, float4* planes, i
     const unsigned q = min(threadIdx.x, plane - 1), xq = q % P;
     const bool on = threadIdx.x < plane, row_end = PAD && xq == P - 1, first = lane == 0, last = lane == 31 || q + 1 == plane;
     const bool fix1 = row_end && rem == 1, fix2 = row_end && rem == 2, fix3 = row_end && rem == 3;
-    const int left = -1 - (PAD && xq == 0 ? 4 - rem : 0);
+    const int left = -1 - (PAD && xq == 0 && rem ? 4 - rem : 0);
     const bool push_low = on && rank > 0, push_high = on && z0 + NZ < S.d;
     const unsigned low = remote_address(planes + (K + 1) * plane + q, max(rank - 1, 0)),
                    high = remote_address(planes + q, rank + (z0 + NZ < S.d ? 1 : 0));
@@ -1130,90 +1130,98 @@ __device__ __forceinline__ void poisson_block(const CdmSeg& S, float4* planes, i
     sweep(kPSweeps & 1 ? 0 : copy, 0, true);
 }
 
-template <int K, bool PAD>
-__global__ void __launch_bounds__(kPClusterThreads) cdm_poisson_cluster_kernel(const __grid_constant__ CdmSeg S)
+// Three clusters an entry.
+template <bool PAD, bool MULTI>
+__global__ void __launch_bounds__(kPClusterThreads) cdm_poisson_cluster_kernel(const CdmSeg* __restrict__ segs,
+                                                                               const __grid_constant__ CdmSeg one)
 {
     extern __shared__ float4 planes[];  // two copies of K + 2 planes
+    const CdmSeg& S = MULTI ? segs[blockIdx.x / (3 * kPCluster)] : one;
     if (S.ctl->done)
         return;
-    const int rank = (int)blockIdx.x % kPCluster, comp = (int)blockIdx.x / kPCluster;
-    const int nz = max(0, min(K, S.d - rank * K));  // the same for every thread of the block
-    if (nz == K)
-        poisson_block<K, PAD>(S, planes, K, rank, comp);
-    else if (K > 3 && nz == 3)
-        poisson_block<3, PAD>(S, planes, K, rank, comp);
-    else if (K > 2 && nz == 2)
-        poisson_block<2, PAD>(S, planes, K, rank, comp);
-    else if (K > 1 && nz == 1)
-        poisson_block<1, PAD>(S, planes, K, rank, comp);
-    else
+    const int rank = (int)blockIdx.x % kPCluster, comp = (int)blockIdx.x / kPCluster % 3;
+    const int K = (S.d + kPCluster - 1) / kPCluster;
+    static_assert(kPClusterPlanes == 4, "one case for each number of planes");
+    switch (max(0, min(K, S.d - rank * K))) {  // the same for every thread of the block
+    case 4: poisson_block<4, PAD>(S, planes, K, rank, comp); break;
+    case 3: poisson_block<3, PAD>(S, planes, K, rank, comp); break;
+    case 2: poisson_block<2, PAD>(S, planes, K, rank, comp); break;
+    case 1: poisson_block<1, PAD>(S, planes, K, rank, comp); break;
+    default:
         for (int k = 0; k < kPSweeps; ++k)
             cluster_barrier();
+    }
 }
 
-// The launch for a level of d <= K * kPCluster planes; cudaErrorNotSupported where the device
-// cannot hold a whole cluster.
-template <int K, bool PAD>
-cudaError_t launch_poisson_cluster(const CdmSeg& s, cudaStream_t st)
-{
-    auto config = [&](unsigned cols, cudaLaunchAttribute& attr) {
+struct ClusterLaunch {
+    cudaLaunchAttribute attr{};
+    cudaLaunchConfig_t cfg{};
+    ClusterLaunch(int n, unsigned cols, unsigned planes, cudaStream_t st)
+    {
         attr.id = cudaLaunchAttributeClusterDimension;
         attr.val.clusterDim.x = kPCluster;
         attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3(3 * kPCluster);
+        cfg.gridDim = dim3(3 * kPCluster * n);
         cfg.blockDim = dim3((cols + 31) / 32 * 32);
-        cfg.dynamicSmemBytes = 2 * (K + 2) * cols * sizeof(float4);
+        cfg.dynamicSmemBytes = 2 * (planes + 2) * cols * sizeof(float4);
         cfg.stream = st;
         cfg.attrs = &attr;
         cfg.numAttrs = 1;
-        return cfg;
-    };
-    cudaLaunchAttribute attr{};
+    }
+};
+
+// Lets the cluster kernels have their shared memory and cluster size on the current device;
+// whether it can hold a whole cluster.
+bool clusters_fit()
+{
     static std::atomic<unsigned long long> asked{0}, fits{0};
     int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess)
-        return e;
+    if (cudaGetDevice(&dev) != cudaSuccess)
+        return false;
     const unsigned long long bit = 1ull << (dev & 63);
     if (!(asked.load() & bit)) {
-        e = cudaFuncSetAttribute(cdm_poisson_cluster_kernel<K, PAD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 2 * (K + 2) * kPClusterThreads * (int)sizeof(float4));
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(cdm_poisson_cluster_kernel<K, PAD>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        int clusters = 0;
-        if (e == cudaSuccess) {
-            const cudaLaunchConfig_t cfg = config(kPClusterThreads, attr);
-            e = cudaOccupancyMaxActiveClusters(&clusters, cdm_poisson_cluster_kernel<K, PAD>, &cfg);
+        const ClusterLaunch most(1, kPClusterThreads, kPClusterPlanes, nullptr);
+        bool ok = true;
+        auto kernels = {cdm_poisson_cluster_kernel<false, false>, cdm_poisson_cluster_kernel<true, false>,
+                        cdm_poisson_cluster_kernel<true, true>};
+        for (auto k : kernels) {
+            int clusters = 0;
+            ok = ok &&
+                 cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most.cfg.dynamicSmemBytes) ==
+                     cudaSuccess &&
+                 cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                 cudaOccupancyMaxActiveClusters(&clusters, k, &most.cfg) == cudaSuccess && clusters > 0;
         }
-        if (e != cudaSuccess)
-            return e;
-        if (clusters > 0)
+        if (ok)
             fits.fetch_or(bit);
         asked.fetch_or(bit);
     }
-    if (!(fits.load() & bit))
-        return cudaErrorNotSupported;
-    const cudaLaunchConfig_t cfg = config((unsigned)(s.ppitch / 4 * s.h), attr);
-    e = cudaLaunchKernelEx(&cfg, cdm_poisson_cluster_kernel<K, PAD>, s);
+    return fits.load() & bit;
+}
+
+bool cdm_poisson_small(const CdmSeg& s)
+{
+    return s.ppitch % 4 == 0 && s.ppitch / 4 * s.h <= kPClusterThreads && s.d <= kPCluster * kPClusterPlanes &&
+           clusters_fit();
+}
+
+// The sweeps of L's first L.small entries.
+cudaError_t launch_poisson_clusters(const CdmSegs& L, cudaStream_t st)
+{
+    unsigned cols = 0, planes = 0;
+    for (int k = 0; k < L.small; ++k) {
+        const CdmSeg& s = L.host[k];
+        cols = std::max(cols, (unsigned)(s.ppitch / 4 * s.h));
+        planes = std::max(planes, (unsigned)((s.d + kPCluster - 1) / kPCluster));
+    }
+    const ClusterLaunch launch(L.small, cols, planes, st);
+    auto kernel = L.small > 1         ? cdm_poisson_cluster_kernel<true, true>
+                  : L.host->w % 4 == 0 ? cdm_poisson_cluster_kernel<false, false>
+                                       : cdm_poisson_cluster_kernel<true, false>;
+    const cudaError_t e = cudaLaunchKernelEx(&launch.cfg, kernel, L.dev, *L.host);
     if (e == cudaSuccess)
         count_launch();
     return e;
-}
-
-// The sweeps of one level in clusters where it fits them, else cudaErrorNotSupported.
-cudaError_t launch_poisson_clusters(const CdmSeg& s, cudaStream_t st)
-{
-    if (s.ppitch % 4 || s.ppitch / 4 * s.h > kPClusterThreads)
-        return cudaErrorNotSupported;
-    static_assert(kPClusterPlanes == 4, "one instantiation for each number of planes");
-    switch ((s.d + kPCluster - 1) / kPCluster) {
-    case 1: return s.w & 3 ? launch_poisson_cluster<1, true>(s, st) : launch_poisson_cluster<1, false>(s, st);
-    case 2: return s.w & 3 ? launch_poisson_cluster<2, true>(s, st) : launch_poisson_cluster<2, false>(s, st);
-    case 3: return s.w & 3 ? launch_poisson_cluster<3, true>(s, st) : launch_poisson_cluster<3, false>(s, st);
-    case 4: return s.w & 3 ? launch_poisson_cluster<4, true>(s, st) : launch_poisson_cluster<4, false>(s, st);
-    default: return cudaErrorNotSupported;
-    }
 }
 
 // An interleaved xyz field to the component planes of a segment's scratch, and back.
@@ -1850,15 +1858,18 @@ cudaError_t launch_cdm_gradient(const CdmSegs& L, int pix, int gradient_type,
 
 cudaError_t launch_cdm_poisson(const CdmSegs& L, cudaStream_t st)
 {
-    if (L.n == 1) {
-        const cudaError_t e = launch_poisson_clusters(*L.host, st);
-        if (e != cudaErrorNotSupported)
+    if (L.small) {
+        const cudaError_t e = launch_poisson_clusters(L, st);
+        if (e != cudaSuccess)
             return e;
     }
+    const int n = L.n - L.small;
+    if (n == 0)
+        return cudaSuccess;
     for (int k = 0; k < kPSweeps; ++k) {
-        auto kernel = L.n > 1 ? (k ? cdm_poisson_kernel<false, true> : cdm_poisson_kernel<true, true>)
-                              : (k ? cdm_poisson_kernel<false, false> : cdm_poisson_kernel<true, false>);
-        kernel<<<L.pblocks, kPThreads, 0, st>>>(L.dev, L.n, *L.host, k & 1);
+        auto kernel = n > 1 ? (k ? cdm_poisson_kernel<false, true> : cdm_poisson_kernel<true, true>)
+                            : (k ? cdm_poisson_kernel<false, false> : cdm_poisson_kernel<true, false>);
+        kernel<<<L.pblocks, kPThreads, 0, st>>>(L.dev + L.small, n, L.host[L.small], k & 1);
     }
     count_launch(kPSweeps);
     return cudaGetLastError();

@@ -106,13 +106,16 @@ struct CdmSeg {
     long long planes_floats() const { return 3 * pplane; }
 };
 // The segments of one launch: n entries on the device and on the host (one entry alone is
-// passed to the kernels by value); blocks / pblocks / tblocks: sum(nblk) / sum(pnb) / sum(tnb)
-// over the entries, whose blk0 / pblk0 / tblk0 number them.
+// passed to the kernels by value).  The first `small` entries are those of cdm_poisson_small,
+// whose sweeps run in clusters.  blocks / tblocks: sum(nblk) / sum(tnb) over the entries, pblocks:
+// sum(pnb) over the others; blk0 / tblk0 / pblk0 number them.
 struct CdmSegs {
     const CdmSeg* dev;
     const CdmSeg* host;
-    int n, blocks, pblocks, tblocks;
+    int n, blocks, pblocks, tblocks, small;
 };
+// Whether the 12 Poisson sweeps of a planar segment run in one launch of clusters.
+bool cdm_poisson_small(const CdmSeg& s);
 // Sets a segment's dims and the launch shapes that follow from them.
 void cdm_set_dims(CdmSeg& s, int w, int h, int d);
 

@@ -72,7 +72,8 @@ void CdmScheduler::loop()
                 segs_.alloc(cap, st_);
                 status_.alloc(cap, st_);
             }
-            // segments sorted into groups of one (pixel type, modality gradient types)
+            // segments sorted into groups of one (pixel type, modality gradient types), the
+            // levels whose Poisson sweeps run in clusters first
             std::vector<int> order(n);
             for (int i = 0; i < n; ++i)
                 order[i] = i;
@@ -80,31 +81,37 @@ void CdmScheduler::loop()
             for (int i = 0; i < n; ++i)
                 keys[i] = std::to_string(cur[i]->lvl->pix) + ":" + cur[i]->lvl->gtypes;
             auto key = [&](int i) -> const std::string& { return keys[i]; };
-            std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return key(a) < key(b); });
+            auto large = [&](int i) { return !cdm_poisson_small(cur[i]->lvl->seg); };
+            std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
+                return key(a) != key(b) ? key(a) < key(b) : large(a) < large(b);
+            });
             for (int i = 0; i < n; ++i)
                 h_segs_.p[i] = cur[order[i]]->lvl->seg;
             // one launch per group over exactly its blocks: each entry's blk0 counts the
             // blocks of the group's entries before it
             struct Group {
-                int g0, g1, blocks, pblocks, tblocks;
+                int g0, g1, blocks, pblocks, tblocks, small;
                 bool first;
             };
             std::vector<Group> groups;
             for (int g0 = 0; g0 < n;) {
-                int g1 = g0, blocks = 0, pblocks = 0, tblocks = 0;
+                int g1 = g0, blocks = 0, pblocks = 0, tblocks = 0, small = 0;
                 bool first = false;
                 while (g1 < n && key(order[g1]) == key(order[g0])) {
                     h_segs_.p[g1].blk0 = blocks;
                     h_segs_.p[g1].pblk0 = pblocks;
                     h_segs_.p[g1].tblk0 = tblocks;
                     blocks += h_segs_.p[g1].nblk;
-                    pblocks += h_segs_.p[g1].pnb;
+                    if (cdm_poisson_small(h_segs_.p[g1]))
+                        ++small;
+                    else
+                        pblocks += h_segs_.p[g1].pnb;
                     tblocks += h_segs_.p[g1].tnb;
                     first = first || !cur[order[g1]]->started;
                     cur[order[g1]]->started = true;
                     ++g1;
                 }
-                groups.push_back({g0, g1, blocks, pblocks, tblocks, first});
+                groups.push_back({g0, g1, blocks, pblocks, tblocks, small, first});
                 g0 = g1;
             }
             REGB_CK(cudaEventRecord(ev_[0], st_));
@@ -112,7 +119,8 @@ void CdmScheduler::loop()
             for (int it = 0; it < iters_; ++it)
                 for (const Group& g : groups) {
                     const Entry* e = cur[order[g.g0]];
-                    launch_iteration(CdmSegs{segs_.p + g.g0, h_segs_.p + g.g0, g.g1 - g.g0, g.blocks, g.pblocks, g.tblocks},
+                    launch_iteration(CdmSegs{segs_.p + g.g0, h_segs_.p + g.g0, g.g1 - g.g0, g.blocks, g.pblocks,
+                                             g.tblocks, g.small},
                                      e->lvl->pix, e->lvl->gtypes, st_, it == 0 && g.first);
                 }
             REGB_CK(launch_cdm_status(segs_.p, n, status_.p, st_));
