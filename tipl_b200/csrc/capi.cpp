@@ -382,15 +382,7 @@ regb_status regb_subject_image_pre(const regb_volume* in, regb_volume* out, void
         Staged a, b;
         a.in(in->ptr, n * pix_size(in->dtype), in->location, st, true);
         b.in(out->ptr, n, out->location, st, false);
-        DevBuf<float> wide;
-        const float* f = (const float*)a.d;
-        if (in->dtype != REGB_F32) {
-            wide.alloc(n, st);
-            REGB_CK(launch_widen_to_f32(a.d, in->dtype, (long long)n, wide.p, st));
-            count_launch();
-            f = wide.p;
-        }
-        subject_image_pre(f, in->dim, (uint8_t*)b.d, st);
+        subject_image_pre(a.d, in->dtype, in->dim, (uint8_t*)b.d, st);
         b.out(out->ptr, st);
         REGB_CK(cudaStreamSynchronize(st));
         return REGB_OK;

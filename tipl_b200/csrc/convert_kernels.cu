@@ -7,42 +7,13 @@
 // ((v - min) * (upper / (max - min)), truncated), with min/max found exactly.
 #include <algorithm>
 #include "kernels.h"
+#include "voxel.cuh"
 
 namespace regb {
 
 namespace {
 
 constexpr int kThreads = 256;
-
-template <int DT>
-__device__ __forceinline__ float load_as_float(const void* p, long long i);
-template <>
-__device__ __forceinline__ float load_as_float<0>(const void* p, long long i)
-{
-    return (float)((const uint8_t*)p)[i];
-}
-template <>
-__device__ __forceinline__ float load_as_float<1>(const void* p, long long i)
-{
-    return ((const float*)p)[i];
-}
-template <>
-__device__ __forceinline__ float load_as_float<2>(const void* p, long long i)
-{
-    return (float)((const uint16_t*)p)[i];
-}
-template <>
-__device__ __forceinline__ float load_as_float<3>(const void* p, long long i)
-{
-    return __uint_as_float((unsigned)((const uint16_t*)p)[i] << 16);
-}
-
-// Order-preserving integer key of a float (for atomicMin/atomicMax).
-__device__ __forceinline__ unsigned key_of(float f)
-{
-    const unsigned u = __float_as_uint(f);
-    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
 
 // mm[0] = min key, mm[1] = max key; mm must hold {0xffffffff, 0} on entry.
 template <int DT>
@@ -71,11 +42,6 @@ __global__ void __launch_bounds__(kThreads) minmax_kernel(const void* __restrict
         atomicMin(&mm[0], lo);
         atomicMax(&mm[1], hi);
     }
-}
-
-__device__ __forceinline__ float float_of(unsigned k)
-{
-    return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
 }
 
 // out[i] = uint8((v[i] - min) * (upper / (max - min))); leaves out untouched when max == min.

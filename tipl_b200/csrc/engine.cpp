@@ -359,14 +359,8 @@ private:
         if (s.subject_pre) {
             // the mm_reg pipeline: the subject through subject_image_pre, the template
             // through template_image_pre (its uint8 copy), both stages on uint8
-            DevBuf<float> wide;
-            const float* f = (const float*)d_moving;
-            if (s.moving.dtype != REGB_F32) {
-                to_f32(d_moving, s.moving.dtype, nm, wide, st.s);
-                f = wide.p;
-            }
             moving_q.alloc(nm, st.s);
-            subject_image_pre(f, s.moving.dim, moving_q.p, st.s);
+            subject_image_pre(d_moving, s.moving.dtype, s.moving.dim, moving_q.p, st.s);
             moving_u8 = moving_q.p;
             if (!fixed_u8) {
                 to_u8(d_fixed, fdtype, nfx, fixed_q, st.s);

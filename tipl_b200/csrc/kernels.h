@@ -191,23 +191,27 @@ cudaError_t launch_minmax(const void* in, int dtype, long long n, unsigned* mm, 
 // Exact widening of a U8 / F32 / U16 / BF16 volume to float.
 cudaError_t launch_widen_to_f32(const void* in, int dtype, long long n, float* out, cudaStream_t st);
 
-// Subject preprocessing (preprocess_kernels.cu).  One round of the separable [1 2 1]
-// Gaussian (x, y, z passes), optionally times scale.
-cudaError_t launch_gaussian_round(const float* in, float* out, int w, int h, int d, float scale, int apply_scale,
-                                  cudaStream_t st);
-// 256-bin histogram of floor((v - mn) * range), clamped to [0, 255] (zeroes hist first).
-cudaError_t launch_otsu_hist(const float* v, long long n, float mn, float range, unsigned* hist, cudaStream_t st);
+// Subject preprocessing (preprocess_kernels.cu); v: 16-byte aligned.  One round of the separable
+// [1 2 1] Gaussian (x, y, z passes) of a U8 / F32 / U16 / BF16 volume, optionally times scale;
+// with mm also the keys of its smallest and largest result (mm = {0xffffffff, 0} on entry).
+cudaError_t launch_gaussian_round(const void* in, int dtype, float* out, int w, int h, int d, float scale,
+                                  int apply_scale, unsigned* mm, cudaStream_t st);
+// Adds to hist the 256-bin histogram of floor((v - min) * (256 / (max - min))), clamped to
+// [0, 255], min and max from their keys; nothing unless min < max.
+cudaError_t launch_otsu_hist(const float* v, long long n, const unsigned* mm, unsigned* hist, cudaStream_t st);
 // The values > ot in voxel order into out; counts holds compact_tiles(n) + 1 words and
 // receives the total in its last word.
 long long compact_tiles(long long n);
 cudaError_t launch_compact_above(const float* v, long long n, float ot, unsigned* counts, float* out, cudaStream_t st);
-// The 256 chunk middles of median() over m >= 2048 values.
-cudaError_t launch_chunk_medians(const float* v, long long m, float* med, cudaStream_t st);
+// The 256 chunk middles of median() over the *count values of v, all above ot and none with a
+// key above *max_key; nothing when there are fewer than 2048.
+cudaError_t launch_chunk_medians(const float* v, const unsigned* count, float ot, const unsigned* max_key, float* med,
+                                 cudaStream_t st);
 // count of v * s > 0 (zeroes cnt first)
 cudaError_t launch_positive_count(const float* v, long long n, float s, unsigned long long* cnt, cudaStream_t st);
-// out = uint8(clamp(v * s - (shift ? c : 0), 0, upper))
-cudaError_t launch_otsu_normalize(const float* v, long long n, float s, int shift, float c, float upper, uint8_t* out,
-                                  cudaStream_t st);
+// out = uint8(clamp(v * s - (shift ? c : 0), 0, upper)), shift: *cnt is more than half of n
+cudaError_t launch_otsu_normalize(const float* v, long long n, float s, const unsigned long long* cnt, float c,
+                                  float upper, uint8_t* out, cudaStream_t st);
 
 // Mapping steps of the mm_reg pipeline (mapping_kernels.cu).  Fields are AoS float xyz.
 // mapping = T(dis + index); out = iT(index) + trilinear(inv_dis, iT(index)) over MD;

@@ -62,6 +62,49 @@ float middle(std::vector<float>& v)
     return v[v.size() / 2];
 }
 
+// segmentation::otsu_median (numerical/otsu.hpp:86-100) of an image whose smallest and largest
+// value have the keys mm_hist[0] and [1]; the 256 words after them are zero.
+float otsu_median(const float* d_img, long long n, unsigned* mm_hist, cudaStream_t st)
+{
+    REGB_CK(launch_otsu_hist(d_img, n, mm_hist, mm_hist + 2, st));
+    count_launch();
+    unsigned h[2 + 256];
+    REGB_CK(cudaMemcpyAsync(h, mm_hist, sizeof(h), cudaMemcpyDeviceToHost, st));
+    REGB_CK(cudaStreamSynchronize(st));
+    const float mn = key_to_float(h[0]), mx = key_to_float(h[1]);
+    // otsu_threshold (numerical/otsu.hpp:59-71) with histogram (basic_op.hpp:1293-1311)
+    float ot = mn;
+    if (mn < mx) {
+        h[2] = 0;
+        ot = otsu_from_hist(h + 2, mn, mx);
+    }
+    // the median of the values above it, in voxel order (otsu.hpp:86-100): the total and the
+    // chunk middles, should there be chunks, come back together
+    const long long nt = compact_tiles(n);
+    DevBuf<unsigned> counts((size_t)nt + 1 + 256, st);
+    DevBuf<float> above((size_t)std::max<long long>(n, 1), st);
+    unsigned* const total = counts.p + nt;
+    REGB_CK(launch_compact_above(d_img, n, ot, counts.p, above.p, st));
+    REGB_CK(launch_chunk_medians(above.p, total, ot, mm_hist + 1, (float*)(total + 1), st));
+    count_launch(4);
+    struct {
+        unsigned m;
+        float med[256];
+    } r;
+    static_assert(sizeof(r) == 257 * sizeof(unsigned), "as on the device");
+    REGB_CK(cudaMemcpyAsync(&r, total, sizeof(r), cudaMemcpyDeviceToHost, st));
+    REGB_CK(cudaStreamSynchronize(st));
+    if (r.m == 0)
+        return ot;
+    std::vector<float> v(r.med, r.med + 256);
+    if (r.m < 2048) {
+        v.resize(r.m);
+        REGB_CK(cudaMemcpyAsync(v.data(), above.p, r.m * sizeof(float), cudaMemcpyDeviceToHost, st));
+        REGB_CK(cudaStreamSynchronize(st));
+    }
+    return middle(v);
+}
+
 }  // namespace
 
 void gaussian(const float* d_in, const int* dim, int bandwidth, float* d_out, cudaStream_t st)
@@ -81,60 +124,10 @@ void gaussian(const float* d_in, const int* dim, int bandwidth, float* d_out, cu
     for (int k = 0; k < bandwidth; ++k) {
         const bool last = (k + 1 == bandwidth);
         float* dst = ((bandwidth - 1 - k) % 2 == 0) ? d_out : tmp.p;
-        REGB_CK(launch_gaussian_round(src, dst, dim[0], dim[1], dim[2], scale, last ? 1 : 0, st));
+        REGB_CK(launch_gaussian_round(src, REGB_F32, dst, dim[0], dim[1], dim[2], scale, last ? 1 : 0, nullptr, st));
         count_launch();
         src = dst;
     }
-}
-
-float otsu_median(const float* d_img, long long n, cudaStream_t st)
-{
-    DevBuf<unsigned> mm(2, st), hist(256, st);
-    REGB_CK(launch_minmax(d_img, REGB_F32, n, mm.p, st));
-    count_launch();
-    unsigned hmm[2];
-    REGB_CK(cudaMemcpyAsync(hmm, mm.p, sizeof(hmm), cudaMemcpyDeviceToHost, st));
-    REGB_CK(cudaStreamSynchronize(st));
-    const float mn = key_to_float(hmm[0]), mx = key_to_float(hmm[1]);
-    // otsu_threshold (numerical/otsu.hpp:59-71) with histogram (basic_op.hpp:1293-1311)
-    float ot = mn;
-    if (mn < mx) {
-        float range = mx - mn;
-        if (range == 0.0f)
-            range = 1.0f;
-        range = 256.0f / range;
-        REGB_CK(launch_otsu_hist(d_img, n, mn, range, hist.p, st));
-        count_launch();
-        unsigned h[256];
-        REGB_CK(cudaMemcpyAsync(h, hist.p, sizeof(h), cudaMemcpyDeviceToHost, st));
-        REGB_CK(cudaStreamSynchronize(st));
-        h[0] = 0;
-        ot = otsu_from_hist(h, mn, mx);
-    }
-    // the median of the values above it, in voxel order (otsu.hpp:86-100)
-    const long long nt = compact_tiles(n);
-    DevBuf<unsigned> counts((size_t)nt + 1, st);
-    DevBuf<float> above((size_t)std::max<long long>(n, 1), st);
-    REGB_CK(launch_compact_above(d_img, n, ot, counts.p, above.p, st));
-    count_launch(3);
-    unsigned m = 0;
-    REGB_CK(cudaMemcpyAsync(&m, counts.p + nt, sizeof(m), cudaMemcpyDeviceToHost, st));
-    REGB_CK(cudaStreamSynchronize(st));
-    if (m == 0)
-        return ot;
-    std::vector<float> v;
-    if (m < 2048) {
-        v.resize(m);
-        REGB_CK(cudaMemcpyAsync(v.data(), above.p, m * sizeof(float), cudaMemcpyDeviceToHost, st));
-    } else {
-        DevBuf<float> med(256, st);
-        REGB_CK(launch_chunk_medians(above.p, m, med.p, st));
-        count_launch();
-        v.resize(256);
-        REGB_CK(cudaMemcpyAsync(v.data(), med.p, 256 * sizeof(float), cudaMemcpyDeviceToHost, st));
-    }
-    REGB_CK(cudaStreamSynchronize(st));
-    return middle(v);
 }
 
 // correlation(x, y) (numerical/statistics.hpp:569-598), or correlation_ygz (:600-619:
@@ -158,26 +151,27 @@ double correlation_u8(const uint8_t* d_x, const uint8_t* d_y, long long n, bool 
     return ((double)h[4] / dn - mx * my) / sd1 / sd2;
 }
 
-void subject_image_pre(const float* d_in, const int* dim, uint8_t* d_out, cudaStream_t st)
+void subject_image_pre(const void* d_in, int dtype, const int* dim, uint8_t* d_out, cudaStream_t st)
 {
     const long long n = (long long)dim[0] * dim[1] * dim[2];
     const float upper = 255.99f;
     DevBuf<float> g((size_t)n, st);
-    gaussian(d_in, dim, 1, g.p, st);
-    const float ot = otsu_median(g.p, n, st);
+    DevBuf<unsigned> mm_hist(2 + 256, st);
+    REGB_CK(cudaMemsetAsync(mm_hist.p, 0xff, sizeof(unsigned), st));
+    REGB_CK(cudaMemsetAsync(mm_hist.p + 1, 0, 257 * sizeof(unsigned), st));
+    // filter::gaussian(I, 1): 1 / 64
+    REGB_CK(launch_gaussian_round(d_in, dtype, g.p, dim[0], dim[1], dim[2], 1.0f / 64.0f, 1, mm_hist.p, st));
+    count_launch();
+    const float ot = otsu_median(g.p, n, mm_hist.p, st);
     // normalize_otsu_median (otsu.hpp:126-135); a zero median leaves the image as it is
     const float s = (ot == 0.0f) ? 1.0f : upper * 0.5f / ot;
-    int shift = 0;
+    DevBuf<unsigned long long> cnt;
     if (ot != 0.0f) {
-        DevBuf<unsigned long long> cnt(1, st);
+        cnt.alloc(1, st);
         REGB_CK(launch_positive_count(g.p, n, s, cnt.p, st));
         count_launch();
-        unsigned long long pos = 0;
-        REGB_CK(cudaMemcpyAsync(&pos, cnt.p, sizeof(pos), cudaMemcpyDeviceToHost, st));
-        REGB_CK(cudaStreamSynchronize(st));
-        shift = ((double)pos > 0.5 * (double)n) ? 1 : 0;
     }
-    REGB_CK(launch_otsu_normalize(g.p, n, s, shift, upper * 0.1f, ot == 0.0f ? 255.0f : upper, d_out, st));
+    REGB_CK(launch_otsu_normalize(g.p, n, s, cnt.p, upper * 0.1f, ot == 0.0f ? 255.0f : upper, d_out, st));
     count_launch();
 }
 
