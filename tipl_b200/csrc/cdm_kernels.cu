@@ -843,6 +843,35 @@ static_assert(kPSweeps % 2 == 0, "the result lands in aux_d");
 // plane, four a thread.
 constexpr int kTThreads = 128, kTile = 4 * kTThreads, kAVox = 2;
 
+// Planes a thread of the sweeps walks, and their grids, for a launch of n levels.  The fewest
+// that let the whole launch be resident at once keep every SM busy to its end; levels that would
+// take more than 12 have several waves anyway and walk 8, which reads a plane of the input 1.25
+// times (a sweep of 91x109x91: 7.3 us with 8, 6.5 with 5, 7.9 with 4, whose blocks are 1.2
+// waves; 128^3: 12.3 / 10.7 with 11; 100x100x120 8.7 / 7.8 with 7; 182x218x182 the same from 7
+// to 14).
+void cdm_set_walk(CdmSeg* s, int n)
+{
+    constexpr long long kResident = 148 * 4;
+    auto blocks = [](const CdmSeg& e, int dz) {
+        const long long cols = (e.ppitch * e.h + 3) / 4;
+        return 3 * ((cols + kPThreads - 1) / kPThreads) * ((e.d + dz - 1) / dz);
+    };
+    int walk = 8;
+    for (int dz = 1; dz <= 12; ++dz) {
+        long long total = 0;
+        for (int k = 0; k < n; ++k)
+            total += blocks(s[k], dz);
+        if (total <= kResident) {
+            walk = dz;
+            break;
+        }
+    }
+    for (int k = 0; k < n; ++k) {
+        s[k].pdz = walk;
+        s[k].pnb = (int)blocks(s[k], walk);
+    }
+}
+
 // Launch shapes that follow from a level's dims alone.
 void cdm_set_dims(CdmSeg& s, int w, int h, int d)
 {
@@ -855,17 +884,7 @@ void cdm_set_dims(CdmSeg& s, int w, int h, int d)
     const long long rows = (long long)h * d, padded = (w + 3LL) / 4 * 4;
     s.ppitch = (4 * padded <= 5LL * w || padded * rows < (1LL << 24)) ? padded : w;
     s.pplane = s.ppitch * rows;
-    // Planes a thread walks: 8 reads a plane of the input 1.25 times, but a level needs two
-    // blocks an SM first (91x109x91 solve: 87 us with 8, 92 with 4; 182x218x182: 613 / 646,
-    // 648 with 16).
-    const long long cols = (s.ppitch * h + 3) / 4, tiles = 3 * ((cols + kPThreads - 1) / kPThreads);
-    s.pdz = 1;
-    for (int dz = 8; dz > 1; dz /= 2)
-        if (tiles * ((d + dz - 1) / dz) >= 148 * 2) {
-            s.pdz = dz;
-            break;
-        }
-    s.pnb = (int)(tiles * ((d + s.pdz - 1) / s.pdz));
+    cdm_set_walk(&s, 1);
     s.tnb = (int)((s.ppitch * h + kTile - 1) / kTile * d);
 }
 
@@ -1526,12 +1545,13 @@ __global__ void __launch_bounds__(kTThreads) cdm_smooth_compose_kernel(SEG_ARGS)
     T* __restrict__ const Js = (T*)S.Js;
     const Dim3 D{S.w, S.h, S.d};
     const unsigned pitch = (unsigned)S.ppitch;
-    const int tiles = S.tnb / D.d, z = tile / tiles, tp = (tile - z * tiles) * kTile;
+    const int tiles = S.tnb / D.d, z = tile / tiles;
+    const unsigned tp = (unsigned)(tile - z * tiles) * kTile;  // the tile's first position in its plane
     const int lane = threadIdx.x & 31, warp = threadIdx.x & ~31;
     __shared__ float4 field[3][kTThreads];
     if ((pitch & 3) == 0) {
         const unsigned P = pitch / 4, plane = P * (unsigned)D.h, total = plane * (unsigned)D.d;
-        const unsigned q = (unsigned)tp / 4 + threadIdx.x, xq = q % P, i = (unsigned)z * plane + q;
+        const unsigned q = tp / 4 + threadIdx.x, xq = q % P, i = (unsigned)z * plane + q;
         const int rem = D.w & 3;
         const bool on = q < plane, row_end = xq == P - 1;
         const bool fix1 = row_end && rem == 1, fix2 = row_end && rem == 2, fix3 = row_end && rem == 3;
@@ -1570,8 +1590,8 @@ __global__ void __launch_bounds__(kTThreads) cdm_smooth_compose_kernel(SEG_ARGS)
         const long long w = D.w, wh = D.wh(), n = D.n();
         for (int k = 0; k < 3; ++k)
             for (int j = 0; j < 4; ++j) {
-                const int p = tp + 4 * warp + 32 * j + lane;
-                const long long i = z * wh + p;
+                const int v = 4 * warp + 32 * j + lane;
+                const long long p = (long long)tp + v, i = z * wh + p;
                 const float* __restrict__ const d = S.tmp_d + k * S.pplane;
                 float* const out = dst + k * S.pplane;
                 if (p >= wh)
@@ -1580,25 +1600,25 @@ __global__ void __launch_bounds__(kTThreads) cdm_smooth_compose_kernel(SEG_ARGS)
                 if (sm == 0.0f)
                     r = out[i];
                 else {
-                    float v = 0.0f;
-                    if (i + 1 < n) v += d[i + 1];
-                    if (i >= 1) v += d[i - 1];
-                    if (i + w < n) v += d[i + w];
-                    if (i >= w) v += d[i - w];
-                    if (i + wh < n) v += d[i + wh];
-                    if (i >= wh) v += d[i - wh];
-                    v *= w_6;
-                    r = d[i] * w_1 + v;
+                    float a = 0.0f;
+                    if (i + 1 < n) a += d[i + 1];
+                    if (i >= 1) a += d[i - 1];
+                    if (i + w < n) a += d[i + w];
+                    if (i >= w) a += d[i - w];
+                    if (i + wh < n) a += d[i + wh];
+                    if (i >= wh) a += d[i - wh];
+                    a *= w_6;
+                    r = d[i] * w_1 + a;
                     out[i] = r;
                 }
-                reinterpret_cast<float*>(field[k])[p - tp] = r;
+                reinterpret_cast<float*>(field[k])[v] = r;
             }
     }
     __syncwarp();
     const bool fast = S.ndim != 2 && narrow(S);
     const SampleGeo G = sample_geo(D);
     const int v0 = 4 * warp + lane;
-    int y = (int)((unsigned)(tp + v0) / pitch), x = (int)((unsigned)(tp + v0) - (unsigned)y * pitch);
+    int y = (int)((tp + v0) / pitch), x = (int)(tp + v0 - (unsigned)y * pitch);
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
         const int v = v0 + 32 * k;

@@ -118,6 +118,8 @@ struct CdmSegs {
 bool cdm_poisson_small(const CdmSeg& s);
 // Sets a segment's dims and the launch shapes that follow from them.
 void cdm_set_dims(CdmSeg& s, int w, int h, int d);
+// The Poisson sweeps' part of it, for a launch of n segments (cdm_set_dims: of one).
+void cdm_set_walk(CdmSeg* s, int n);
 
 template <typename T>
 cudaError_t launch_resample(const T* from, Dim3 fd, T* to, Dim3 td, const float* Tm, const int* shift,

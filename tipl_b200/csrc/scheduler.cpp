@@ -97,19 +97,19 @@ void CdmScheduler::loop()
             for (int g0 = 0; g0 < n;) {
                 int g1 = g0, blocks = 0, pblocks = 0, tblocks = 0, small = 0;
                 bool first = false;
-                while (g1 < n && key(order[g1]) == key(order[g0])) {
+                while (g1 < n && key(order[g1]) == key(order[g0]))
+                    small += !large(order[g1++]);
+                cdm_set_walk(h_segs_.p + g0 + small, g1 - g0 - small);
+                for (g1 = g0; g1 < n && key(order[g1]) == key(order[g0]); ++g1) {
                     h_segs_.p[g1].blk0 = blocks;
                     h_segs_.p[g1].pblk0 = pblocks;
                     h_segs_.p[g1].tblk0 = tblocks;
                     blocks += h_segs_.p[g1].nblk;
-                    if (cdm_poisson_small(h_segs_.p[g1]))
-                        ++small;
-                    else
+                    if (g1 >= g0 + small)
                         pblocks += h_segs_.p[g1].pnb;
                     tblocks += h_segs_.p[g1].tnb;
                     first = first || !cur[order[g1]]->started;
                     cur[order[g1]]->started = true;
-                    ++g1;
                 }
                 groups.push_back({g0, g1, blocks, pblocks, tblocks, small, first});
                 g0 = g1;
