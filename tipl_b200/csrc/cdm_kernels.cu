@@ -832,10 +832,10 @@ __device__ __forceinline__ bool last_block_of_segment(const CdmSeg& S)
 // Positions outside the field count as +0, whose subtraction changes nothing, like the taps
 // the reference skips.
 //
-// Bound by L2 (and its latency on small levels): 91x109x91, 12 sweeps replayed by a graph, 137
-// us with a thread per float of the interleaved field (nine scalar loads each, the
-// neighbouring rows and planes from L2), 87 so; 182x218x182 1240 / 613, 46x55x46 49 / 40,
-// 23x28x23 40 / 28.
+// Bound by L2 (and its latency): a sweep with a thread per float of the interleaved field (nine
+// scalar loads each, the neighbouring rows and planes from L2), and so: 91x109x91 11.4 / 6.5 us,
+// 128^3 22.7 / 10.7, 182x218x182 103 / 53.  Levels of up to 64 planes of 1024 columns take the
+// clusters below instead (46x55x46, 12 sweeps: 49 / 40 / 17.6).
 constexpr int kPThreads = 256;
 constexpr int kPSweeps = 12;  // reg/cdm.hpp:165
 static_assert(kPSweeps % 2 == 0, "the result lands in aux_d");
@@ -1042,8 +1042,9 @@ __global__ void __launch_bounds__(kPThreads, 4) cdm_poisson_kernel(SEG_ARGS, int
 // ends it.  Taps, padding and arithmetic are poisson_walk's; a halo outside the field stays
 // zero.
 //
-// Bound by the barrier and the exchange (0.65 us a sweep at 16^3) on the smallest, then by issue.  Twelve launches of a sweep before, one so: 23x28x23 25 / 8.8
-// us, 32^3 24.6 / 10.8, 46x55x46 40 / 19, 64^3 40 / 32, and the gaps between the launches.
+// Bound by the barrier and the exchange (0.6 us a sweep at 16^3) on the smallest, then by issue.
+// Twelve launches of a sweep before, one so: 23x28x23 25 / 8.4 us, 32^3 24.6 / 10.9, 46x55x46
+// 40 / 17.6, 64^3 40 / 29, and the gaps between the launches.
 // Larger levels do not fit: a plane has to be a block's columns, 16 blocks hold 64 planes.
 constexpr int kPCluster = 16, kPClusterThreads = 1024, kPClusterPlanes = 4;
 
