@@ -187,15 +187,13 @@ cudaError_t launch_cdm_status(const CdmSeg* segs, int nseg, int* out, cudaStream
 // (then mm[0] == mm[1] afterwards).
 cudaError_t launch_normalize_to_u8(const void* in, int dtype, long long n, float upper, uint8_t* out, unsigned* mm,
                                    cudaStream_t st);
-// Exact min / max of a U8 / F32 / U16 / BF16 volume as order-preserving float keys:
-// mm[0] = key(min), mm[1] = key(max), key(f) = f >= 0 ? bits | 2^31 : ~bits.
-cudaError_t launch_minmax(const void* in, int dtype, long long n, unsigned* mm, cudaStream_t st);
 // Exact widening of a U8 / F32 / U16 / BF16 volume to float.
 cudaError_t launch_widen_to_f32(const void* in, int dtype, long long n, float* out, cudaStream_t st);
 
 // Subject preprocessing (preprocess_kernels.cu); v: 16-byte aligned.  One round of the separable
 // [1 2 1] Gaussian (x, y, z passes) of a U8 / F32 / U16 / BF16 volume, optionally times scale;
-// with mm also the keys of its smallest and largest result (mm = {0xffffffff, 0} on entry).
+// with mm also the order-preserving keys of its smallest and largest result (key(f) = f >= 0 ?
+// bits | 2^31 : ~bits; mm = {0xffffffff, 0} on entry).
 cudaError_t launch_gaussian_round(const void* in, int dtype, float* out, int w, int h, int d, float scale,
                                   int apply_scale, unsigned* mm, cudaStream_t st);
 // Adds to hist the 256-bin histogram of floor((v - min) * (256 / (max - min))), clamped to
