@@ -51,6 +51,8 @@ void CdmScheduler::run(CdmLevel& lvl, volatile const int* terminated)
     active_.push_back(&e);
     cv_.notify_all();
     cv_done_.wait(lk, [&] { return e.done; });
+    if (e.error)
+        std::rethrow_exception(e.error);
 }
 
 void CdmScheduler::loop()
@@ -62,7 +64,7 @@ void CdmScheduler::loop()
             return;
         std::vector<Entry*> cur(active_);
         lk.unlock();
-        bool failed = false;
+        std::exception_ptr failed;
         try {
             const int n = (int)cur.size();
             if ((int)h_segs_.n < n || (int)segs_.n < n || (int)h_status_.n < n || (int)status_.n < n) {
@@ -142,12 +144,15 @@ void CdmScheduler::loop()
                 }
             }
         } catch (...) {
-            failed = true;
+            failed = std::current_exception();
+            // what the round has launched still uses the levels' buffers, which go with their jobs
+            (void)cudaStreamSynchronize(st_);
             lk.lock();
         }
         if (failed) {
-            // leave every level that was in the failed round; its job reads the state
+            // every level that was in the failed round ends with its error
             for (Entry* e : cur) {
+                e->error = failed;
                 e->done = true;
                 auto it = std::find(active_.begin(), active_.end(), e);
                 if (it != active_.end())

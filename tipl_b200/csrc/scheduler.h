@@ -1,6 +1,7 @@
 // Cross-job batching of CDM iterations (the serving engine's nonlinear stage).
 #pragma once
 #include <condition_variable>
+#include <exception>
 #include <mutex>
 #include <thread>
 #include <vector>
@@ -20,7 +21,8 @@ public:
     ~CdmScheduler();
     CdmScheduler(const CdmScheduler&) = delete;
     CdmScheduler& operator=(const CdmScheduler&) = delete;
-    // Iterates the level until its loop ends (or terminated is set); blocks the caller.
+    // Iterates the level until its loop ends (or terminated is set); blocks the caller.  Throws
+    // what ended a round that the level was in.
     void run(CdmLevel& lvl, volatile const int* terminated);
     // counters, read under the scheduler's lock
     long long rounds()
@@ -50,6 +52,7 @@ private:
         volatile const int* term;
         bool done = false;
         bool started = false;  // some round has run its first iteration
+        std::exception_ptr error;  // what ended its round
     };
     void loop();
     std::mutex m_;
