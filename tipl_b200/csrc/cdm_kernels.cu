@@ -1196,8 +1196,10 @@ bool clusters_fit()
 {
     static std::atomic<unsigned long long> asked{0}, fits{0};
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess)
+    if (cudaGetDevice(&dev) != cudaSuccess) {
+        (void)cudaGetLastError();
         return false;
+    }
     const unsigned long long bit = 1ull << (dev & 63);
     if (!(asked.load() & bit)) {
         const ClusterLaunch most(1, kPClusterThreads, kPClusterPlanes, nullptr);
@@ -1214,6 +1216,8 @@ bool clusters_fit()
         }
         if (ok)
             fits.fetch_or(bit);
+        else
+            (void)cudaGetLastError();  // a "no" is an answer: the next launch is not to report it
         asked.fetch_or(bit);
     }
     return fits.load() & bit;
