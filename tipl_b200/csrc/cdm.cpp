@@ -68,7 +68,8 @@ void GraphExec::reset()
 }
 
 void CdmLevel::init(const void* const* It_, const void* const* Is_, const std::string& gtypes_, int w, int h, int d,
-                    int pix_, const regb_cdm_param& p, const float* best, cudaStream_t st, int ndim)
+                    int pix_, const regb_cdm_param& p, const float* best, cudaStream_t st, int ndim,
+                    DevBuf<float>* spent)
 {
     pix = pix_;
     gtypes = gtypes_;
@@ -81,9 +82,12 @@ void CdmLevel::init(const void* const* It_, const void* const* Is_, const std::s
         seg.It[m] = It_[m];
         seg.Is[m] = Is_[m];
     }
+    field[1].alloc(seg.planes_floats(), st);
+    REGB_CK(launch_planes_from_xyz(best, seg, field[1].p, st));  // cur_d(best_d)
+    if (spent)
+        spent->reset();
+    field[0].alloc(seg.planes_floats(), st);
     js.alloc((size_t)n * (pix ? 4 : 1), st);
-    for (int k = 0; k < 2; ++k)
-        field[k].alloc(seg.planes_floats(), st);
     nd.alloc(seg.planes_floats(), st);
     aux.alloc(seg.planes_floats(), st);
     tmp.alloc(seg.planes_floats(), st);
@@ -108,7 +112,6 @@ void CdmLevel::init(const void* const* It_, const void* const* Is_, const std::s
     c.cur = c.from = c.best = 1;
     h_ctl = c;
     REGB_CK(cudaMemcpyAsync(ctl.p, &h_ctl, sizeof(CdmCtl), cudaMemcpyHostToDevice, st));
-    REGB_CK(launch_planes_from_xyz(best, seg, field[1].p, st));  // cur_d(best_d)
     d_seg.alloc(1, st);
     REGB_CK(cudaMemcpyAsync(d_seg.p, &seg, sizeof(CdmSeg), cudaMemcpyHostToDevice, st));
     REGB_CK(cudaStreamSynchronize(st));  // h_ctl / seg are stack-staged: keep the copies ordered before reuse
@@ -244,16 +247,16 @@ regb_status cdm_register_multi(const void* const* d_It, const void* const* d_Is,
         if (k == top)
             REGB_CK(cudaMemsetAsync(best, 0, sizeof(float) * 3 * n, st));
         else {
-            const Lv& C = lv[k + 1];
-            const float* cb = C.best.p;
-            REGB_CK(launch_upsample_field_x2(cb, C.w, C.h, C.d, best, L.w, L.h, L.d, st, ndim));
+            Lv& C = lv[k + 1];
+            REGB_CK(launch_upsample_field_x2(C.best.p, C.w, C.h, C.d, best, L.w, L.h, L.d, st, ndim));
+            C.best.reset();
             if (L.resolution > 1.0f)
                 continue;  // reg/cdm.hpp:404-405
         }
         if (status != REGB_OK)
             continue;
         CdmLevel run;
-        run.init(L.It, L.Is, gtypes, L.w, L.h, L.d, pix, p, best, st, ndim);
+        run.init(L.It, L.Is, gtypes, L.w, L.h, L.d, pix, p, best, st, ndim, &L.best);
         if (sched) {
             // batched with the other jobs' levels; the scheduler returns once this
             // level's loop has ended
@@ -288,7 +291,12 @@ regb_status cdm_register_multi(const void* const* d_It, const void* const* d_Is,
                     break;
             }
         }
-        run.best_field(best, st);
+        if (k > 0) {
+            // a buffer that the level has no more use for: its result takes no memory beside it
+            run.best_field(run.nd.p, st);
+            L.best = std::move(run.nd);
+        } else
+            run.best_field(d_field, st);
         iters += run.h_ctl.iters_run;
         count_cdm_level(run.h_ctl.iters_run, (long long)n, pix ? 4 : 1);
         if (run.h_ctl.done == 2)

@@ -30,10 +30,12 @@ struct CdmLevel {
     DevBuf<CdmCtl> ctl;
     DevBuf<CdmSeg> d_seg;
     // It / Is: gtypes.size() modality pairs of one shape.  best is the field the level starts
-    // from (the upsampled coarser result).
+    // from (the upsampled coarser result); the level takes its own copy of it before it
+    // allocates the rest, and lets spent go then.
     // ndim 2: a level of a 2-D registration (d == 1).
     void init(const void* const* It, const void* const* Is, const std::string& gtypes, int w, int h, int d, int pix,
-              const regb_cdm_param& p, const float* best, cudaStream_t st, int ndim = 3);
+              const regb_cdm_param& p, const float* best, cudaStream_t st, int ndim = 3,
+              DevBuf<float>* spent = nullptr);
     // The best field as of h_ctl, interleaved.
     void best_field(float* xyz, cudaStream_t st) const;
 };
