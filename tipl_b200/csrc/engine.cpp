@@ -226,7 +226,7 @@ private:
         if (j.moving.dtype != REGB_U8 || j.subject_pre)
             b += nm;                          // uint8 copy for the affine stage
         if (j.subject_pre)
-            b += 12.0 * nm;                   // widened copy, smoothed copy, values above the threshold
+            b += 8.0 * nm;                    // smoothed copy, values above the threshold
         if (j.template_id < 0 && ftype != REGB_U8)
             b += nf;
         if (j.run_cdm && float_cdm)
@@ -234,15 +234,18 @@ private:
         if (j.run_linear)
             b += 0.15 * (nf + nm);
         if (j.run_cdm) {
-            b += nf * (float_cdm ? 4.0 : ps) + 12.0 * nf;  // resampled subject, output field
-            // the largest iterated level: 5 fields + composed image
+            const double px = float_cdm ? 4.0 : 1.0;
+            b += nf * px + 12.0 * nf;  // resampled subject, output field
+            // the largest iterated level: 5 fields of padded rows (CdmLevel) + composed image
             int w = fd[0], h = fd[1], d = fd[2];
             float res = j.cdm.resolution;
             double worst = 0.0;
             std::vector<double> lv;
             std::vector<float> lr;
             for (;;) {
-                lv.push_back((double)w * h * d);
+                CdmSeg seg{};
+                cdm_set_dims(seg, w, h, d);
+                lv.push_back(5.0 * sizeof(float) * (double)seg.planes_floats() + px * w * h * d);
                 lr.push_back(res);
                 if (!((unsigned)std::min(w, std::min(h, d)) > j.cdm.min_dimension))
                     break;
@@ -254,9 +257,9 @@ private:
             for (size_t k = 0; k < lv.size(); ++k)
                 if (k + 1 == lv.size() || lr[k] <= 1.0f)
                     worst = std::max(worst, lv[k]);
-            b += worst * (60.0 + ps) + 0.3 * nf * ps;
+            b += worst + 0.3 * nf * px;
             if (j.mm_reg)  // the reverse CDM, the mappings, the composed subject
-                b += worst * (60.0 + ps) + 0.3 * nf * ps + 12.0 * nf + 12.0 * nf + 12.0 * nm + 2.0 * nf;
+                b += worst + 0.3 * nf * px + 12.0 * nf + 12.0 * nf + 12.0 * nm + 2.0 * nf;
         }
         return (size_t)b + (16u << 20);
     }
