@@ -249,6 +249,8 @@ private:
                 lr.push_back(res);
                 if (!((unsigned)std::min(w, std::min(h, d)) > j.cdm.min_dimension))
                     break;
+                if (w == 1 && h == 1 && d == 1)  // only min_dimension 0 gets here (cdm_register_multi)
+                    throw Failure(REGB_ERR_ARG, "cdm: min_dimension 0 never stops downsampling");
                 w = (w + 1) / 2;
                 h = (h + 1) / 2;
                 d = (d + 1) / 2;
