@@ -29,3 +29,19 @@ def test_failed_cluster_check_leaves_no_error(shapes):
     assert (used, error) == (1, 0) and calls > 1
     for k in range(1, calls + 1):
         assert shapes("probe", k)[:2] == [0, 0]
+
+
+# (x, y, z): the grids of templates and subjects, long and flat volumes, rows of a few voxels
+DIMS = [(91, 109, 91), (182, 218, 182), (128, 128, 128), (68, 66, 70), (4, 4, 20000), (8, 8, 5000), (16, 16, 1500),
+        (24, 24, 800), (36, 32, 400), (1, 300, 300), (2, 300, 300), (3, 300, 300), (300, 300, 3), (300, 1, 1000),
+        (200000, 1, 1), (1, 200000, 1), (2, 200000, 1), (1, 1, 200000), (1, 300, 1000)]
+
+
+@pytest.mark.parametrize("dims", DIMS)
+def test_poisson_threads_have_work(shapes, dims):
+    """The sweeps' threads have places for at most twice the padded voxels (four a place), but for
+    a block a component; and padded rows take at most 60 % more than their voxels (5 of 8)."""
+    pitch, plane, _, pnb, pdz, _ = shapes("dims", *dims)
+    assert pnb * 256 * max(pdz, 1) <= 2 * 3 * (plane / 4) + 3 * 256 * max(pdz, 1)
+    n = dims[0] * dims[1] * dims[2]
+    assert plane <= 1.6 * n and pitch * dims[1] * dims[2] == plane

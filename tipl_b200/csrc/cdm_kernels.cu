@@ -843,18 +843,36 @@ static_assert(kPSweeps % 2 == 0, "the result lands in aux_d");
 // plane, four a thread.
 constexpr int kTThreads = 128, kTile = 4 * kTThreads, kAVox = 2;
 
+// The clusters of small levels (below): a block's columns are a plane's, and its planes few.
+constexpr int kPCluster = 16, kPClusterThreads = 1024, kPClusterPlanes = 4;
+static bool cluster_holds(long long pitch, int h, int d)
+{
+    return pitch / 4 * h <= kPClusterThreads && d <= kPCluster * kPClusterPlanes;
+}
+
 // Planes a thread of the sweeps walks, and their grids, for a launch of n levels.  The fewest
 // that let the whole launch be resident at once keep every SM busy to its end; levels that would
 // take more than 12 have several waves anyway and walk 8, which reads a plane of the input 1.25
 // times (a sweep of 91x109x91: 7.3 us with 8, 6.5 with 5, 7.9 with 4, whose blocks are 1.2
 // waves; 128^3: 12.3 / 10.7 with 11; 100x100x120 8.7 / 7.8 with 7; 182x218x182 the same from 7
 // to 14).
+//
+// Planes that leave more than a fifth of their blocks' threads without a column, and single
+// planes, are not walked: the threads take the component's float4 one after the other, the z taps
+// from L1 (12 sweeps walked / so: 4x4x20000 744 / 46 us, 16x16x1500 90 / 52, 36x32x400, 56 % of
+// the threads, 75 / 59; 28x28x700, 77 %, the same; 44x44x300, 95 %, 66 / 69).
 void cdm_set_walk(CdmSeg* s, int n)
 {
     constexpr long long kResident = 148 * 4;
-    auto blocks = [](const CdmSeg& e, int dz) {
-        const long long cols = (e.ppitch * e.h + 3) / 4;
-        return 3 * ((cols + kPThreads - 1) / kPThreads) * ((e.d + dz - 1) / dz);
+    auto blocks_of = [](long long items) { return (items + kPThreads - 1) / kPThreads; };
+    auto whole = [&](const CdmSeg& e) {
+        const long long cols = e.ppitch / 4 * e.h;
+        return (e.ppitch & 3) || e.d == 1 || 5 * cols < 4 * blocks_of(cols) * kPThreads;
+    };
+    auto blocks = [&](const CdmSeg& e, int dz) {
+        if (e.ppitch & 3)  // four floats a thread (2x200000x1: 74 us, one a thread 114)
+            return 3 * blocks_of((e.pplane + 3) / 4);
+        return 3 * (whole(e) ? blocks_of(e.pplane / 4) : blocks_of(e.ppitch / 4 * e.h) * ((e.d + dz - 1) / dz));
     };
     int walk = 8;
     for (int dz = 1; dz <= 12; ++dz) {
@@ -867,7 +885,7 @@ void cdm_set_walk(CdmSeg* s, int n)
         }
     }
     for (int k = 0; k < n; ++k) {
-        s[k].pdz = walk;
+        s[k].pdz = whole(s[k]) ? 0 : walk;
         s[k].pnb = (int)blocks(s[k], walk);
     }
 }
@@ -879,10 +897,14 @@ void cdm_set_dims(CdmSeg& s, int w, int h, int d)
     s.h = h;
     s.d = d;
     s.nblk = cdm_blocks_for((long long)w * h * d);
-    // component planes of new_d / aux_d / tmp_d: rows padded to 4 voxels, unless that costs
-    // memory that counts (very short rows of a huge volume)
+    // component planes of the fields: rows padded to 4 voxels, unless that doubles them (rows of
+    // one or two voxels; not where the sweeps then run in clusters) or costs memory that counts
+    // (other short rows of a huge volume).  12 sweeps with padded rows / so: 1x200000x1 86 / 48
+    // us, 2x200000x1 86 / 74, 2x300x300 50 / 48, but 3x300x300 50 / 64.
     const long long rows = (long long)h * d, padded = (w + 3LL) / 4 * 4;
-    s.ppitch = (4 * padded <= 5LL * w || padded * rows < (1LL << 24)) ? padded : w;
+    const bool pad = 4 * padded <= 5LL * w || cluster_holds(padded, h, d) ||
+                     (padded < 2LL * w && padded * rows < (1LL << 24));
+    s.ppitch = pad ? padded : w;
     s.pplane = s.ppitch * rows;
     cdm_set_walk(&s, 1);
     s.tnb = (int)((s.ppitch * h + kTile - 1) / kTile * d);
@@ -913,17 +935,18 @@ __device__ __forceinline__ float load_now(const float* __restrict__ p, bool ok)
     return f;
 }
 
-// One block's part of a sweep: float4 column q of a plane, planes [z0, z1).  FIRST: the input
-// is the right-hand side times c6.  EDGE: some tap of the block may lie outside the field.
+// One block's part of a sweep: float4 column q of the `span` that its threads' columns are taken
+// from (a plane, or the whole component for planes [0, 1)), planes [z0, z1).  FIRST: the input is
+// the right-hand side times c6.  EDGE: some tap of the block may lie outside the field.
 template <bool FIRST, bool EDGE>
 __device__ __forceinline__ void poisson_walk(const CdmSeg& S, const float4* __restrict__ in, const float4* __restrict__ rhs,
-                                             float4* __restrict__ out, unsigned q, int z0, int z1, int done)
+                                             float4* __restrict__ out, unsigned q, unsigned span, int z0, int z1, int done)
 {
     const unsigned P = (unsigned)(S.ppitch / 4), plane = P * (unsigned)S.h, total = plane * (unsigned)S.d;
     const float c6 = poisson_weight(S);
     const int rem = S.w & 3, lane = threadIdx.x & 31;
     const unsigned xq = q % P;
-    const bool on = q < plane, row_end = xq == P - 1;
+    const bool on = q < span, row_end = xq == P - 1;
     const bool fix1 = row_end && rem == 1, fix2 = row_end && rem == 2, fix3 = row_end && rem == 3;
     unsigned i = (unsigned)z0 * plane + q;
     auto inside = [&](unsigned k) { return on && (!EDGE || k < total); };
@@ -965,7 +988,7 @@ __device__ __forceinline__ void poisson_walk(const CdmSeg& S, const float4* __re
         float xl = __shfl_up_sync(0xffffffffu, tail, 1), xr = __shfl_down_sync(0xffffffffu, cur.x, 1);
         if (lane == 0)
             xl = one(4LL * i - 1 - (xq == 0 && rem ? 4 - rem : 0));
-        if (lane == 31 || q + 1 == plane)
+        if (lane == 31 || q + 1 == span)
             xr = one(4LL * i + 4);
         const float n1 = fix1 ? xr : cur.y, n2 = fix2 ? xr : cur.z, n3 = fix3 ? xr : cur.w;
         float4 v;
@@ -1021,16 +1044,22 @@ __global__ void __launch_bounds__(kPThreads, 4) cdm_poisson_kernel(SEG_ARGS, int
         if (!done)
             poisson_flat<FIRST>(S, in, rhs, out, t, per);
     } else {
-        const int nz = (S.d + S.pdz - 1) / S.pdz, nq = per / nz;
-        const int z0 = t / nq * S.pdz, z1 = min(S.d, z0 + S.pdz);
-        const unsigned q = (unsigned)(t % nq) * kPThreads + threadIdx.x;
+        const unsigned plane = (unsigned)(S.ppitch / 4) * (unsigned)S.h;
         const float4* const in4 = reinterpret_cast<const float4*>(in);
         const float4* const rhs4 = reinterpret_cast<const float4*>(rhs);
         float4* const out4 = reinterpret_cast<float4*>(out);
+        if (S.pdz == 0) {
+            const unsigned q = (unsigned)t * kPThreads + threadIdx.x;
+            poisson_walk<FIRST, true>(S, in4, rhs4, out4, q, plane * (unsigned)S.d, 0, 1, done);
+            return;
+        }
+        const int nz = (S.d + S.pdz - 1) / S.pdz, nq = per / nz;
+        const int z0 = t / nq * S.pdz, z1 = min(S.d, z0 + S.pdz);
+        const unsigned q = (unsigned)(t % nq) * kPThreads + threadIdx.x;
         if (z0 == 0 || z1 == S.d)  // (a plane below and above covers the rows and voxels beside)
-            poisson_walk<FIRST, true>(S, in4, rhs4, out4, q, z0, z1, done);
+            poisson_walk<FIRST, true>(S, in4, rhs4, out4, q, plane, z0, z1, done);
         else
-            poisson_walk<FIRST, false>(S, in4, rhs4, out4, q, z0, z1, done);
+            poisson_walk<FIRST, false>(S, in4, rhs4, out4, q, plane, z0, z1, done);
     }
 }
 
@@ -1046,8 +1075,6 @@ __global__ void __launch_bounds__(kPThreads, 4) cdm_poisson_kernel(SEG_ARGS, int
 // Twelve launches of a sweep before, one so: 23x28x23 25 / 8.4 us, 32^3 24.6 / 10.9, 46x55x46
 // 40 / 17.6, 64^3 40 / 29, and the gaps between the launches.
 // Larger levels do not fit: a plane has to be a block's columns, 16 blocks hold 64 planes.
-constexpr int kPCluster = 16, kPClusterThreads = 1024, kPClusterPlanes = 4;
-
 __device__ __forceinline__ void cluster_barrier()
 {
     __syncwarp();
@@ -1225,8 +1252,7 @@ bool clusters_fit()
 
 bool cdm_poisson_small(const CdmSeg& s)
 {
-    return s.ppitch % 4 == 0 && s.ppitch / 4 * s.h <= kPClusterThreads && s.d <= kPCluster * kPClusterPlanes &&
-           clusters_fit();
+    return s.ppitch % 4 == 0 && cluster_holds(s.ppitch, s.h, s.d) && clusters_fit();
 }
 
 // The sweeps of L's first L.small entries.

@@ -94,8 +94,8 @@ struct CdmSeg {
     // this segment owns blocks [blk0, blk0 + nblk), blk0 ascending along the entries
     // (0 for a launch of this segment alone).
     int blk0;
-    // The Poisson launches' own grid: pnb blocks, pdz planes a thread; pblk0 numbers them as
-    // blk0 does.
+    // The Poisson launches' own grid: pnb blocks, pdz planes a thread (0: the component's float4
+    // one after the other); pblk0 numbers them as blk0 does.
     int pblk0, pnb, pdz;
     // and the grid of an iteration's last two launches (accumulate, smooth and compose)
     int tblk0, tnb;
