@@ -45,3 +45,10 @@ def test_poisson_threads_have_work(shapes, dims):
     assert pnb * 256 * max(pdz, 1) <= 2 * 3 * (plane / 4) + 3 * 256 * max(pdz, 1)
     n = dims[0] * dims[1] * dims[2]
     assert plane <= 1.6 * n and pitch * dims[1] * dims[2] == plane
+
+
+@pytest.mark.parametrize("dims", DIMS)
+def test_tail_blocks_have_work(shapes, dims):
+    """The tail launches have a block for each 512 places of a component."""
+    _, plane, _, _, _, tnb = shapes("dims", *dims)
+    assert 512 * (tnb - 1) < plane <= 512 * tnb

@@ -22,3 +22,24 @@ def test_poisson_thin(orc, shape):
     d[rng.random(shape) < 0.3] = 0
     d[rng.random(shape) < 0.1] = -0.0
     assert np.array_equal(tb.cdm_poisson(d).view(np.uint32), orc.cdm_poisson(d).view(np.uint32))
+
+
+# one level each (no axis is longer than min_dimension); rows of two voxels are not padded
+LEVELS = [(70, 8, 8), (70, 33, 2), (66, 7, 2), (70, 3, 5), (300, 2, 4), (150, 2, 2), (2, 1100, 2), (65, 2, 300), (3, 2, 700),
+          (66, 28, 28), (40, 40, 40)]
+
+
+@pytest.mark.parametrize("gtype", ["r", "d"])
+@pytest.mark.parametrize("u8", [True, False])
+@pytest.mark.parametrize("shape", LEVELS)
+def test_levels_of_thin_volumes(orc, shape, u8, gtype):
+    """Whole levels of random images."""
+    rng = np.random.default_rng(sum(shape))
+    a = rng.random(shape)
+    It, Is = (a * 255), (np.clip(a + rng.normal(0, 0.2, shape), 0, 1) * 255)
+    It, Is = It.astype(np.uint8 if u8 else np.float32), Is.astype(np.uint8 if u8 else np.float32)
+    kw = dict(resolution=1.0, min_dimension=64, gradient_type=gtype)
+    d, ok = tb.reg.cdm(It, Is, tb.reg.cdm_param(**kw))
+    od, ook, _ = orc.cdm(It, Is, **kw)
+    assert ok == ook
+    assert np.array_equal(d.view(np.uint32), od.view(np.uint32))

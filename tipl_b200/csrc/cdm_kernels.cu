@@ -839,8 +839,8 @@ __device__ __forceinline__ bool last_block_of_segment(const CdmSeg& S)
 constexpr int kPThreads = 256;
 constexpr int kPSweeps = 12;  // reg/cdm.hpp:165
 static_assert(kPSweeps % 2 == 0, "the result lands in aux_d");
-// The tail launches (accumulate, smooth and compose): a block takes kTile positions of one
-// plane, four a thread.
+// The tail launches (accumulate, smooth and compose): a block takes kTile positions of a
+// component, whatever rows and planes they belong to.
 constexpr int kTThreads = 128, kTile = 4 * kTThreads, kAVox = 2;
 
 // The clusters of small levels (below): a block's columns are a plane's, and its planes few.
@@ -907,7 +907,7 @@ void cdm_set_dims(CdmSeg& s, int w, int h, int d)
     s.ppitch = pad ? padded : w;
     s.pplane = s.ppitch * rows;
     cdm_set_walk(&s, 1);
-    s.tnb = (int)((s.ppitch * h + kTile - 1) / kTile * d);
+    s.tnb = (int)((s.pplane + kTile - 1) / kTile);
 }
 
 // inv_d2 = -0.5 / dimension (reg/cdm.hpp:163,175): -1/6 in 3-D, -1/4 in 2-D.  A 2-D
@@ -1433,9 +1433,33 @@ __global__ void __launch_bounds__(kCdmThreads) cdm_accumulate_xyz_kernel(SEG_ARG
     }
 }
 
+// The voxel at position p of a component, and the one `step` positions on.
+struct Place {
+    int x, y, z;
+    __device__ __forceinline__ Place(unsigned p, unsigned pitch, int h)
+    {
+        const unsigned r = p / pitch;
+        x = (int)(p - r * pitch);
+        z = (int)(r / (unsigned)h);
+        y = (int)r - z * h;
+    }
+    __device__ __forceinline__ void advance(unsigned step, unsigned pitch, int h)
+    {
+        const unsigned rows = step / pitch;
+        x += (int)(step - rows * pitch);
+        y += (int)rows;
+        if (x >= (int)pitch) {
+            x -= (int)pitch;
+            ++y;
+        }
+        for (; y >= h; y -= h)
+            ++z;
+    }
+};
+
 // Component planes: 24 gathers a voxel, whose lanes take neighbouring floats.  Bound by the
 // chain flag -> update -> cell -> gathers and the L2 traffic of the corner planes; a block
-// takes kTile positions of one plane, so that the last wave of a launch is short.
+// takes kTile positions, so that the last wave of a launch is short.
 // 91x109x91: 14.5 us on interleaved fields with a grid-wide stride, 11.7 so; with 1 / 4 voxels
 // a thread 14.9 / 12.4, 32^3 3.5 us against 2.8 / 6.0.
 constexpr int kAThreads = kTile / kAVox, kABlocks = 1280 / kAThreads;
@@ -1448,19 +1472,18 @@ __global__ void __launch_bounds__(kAThreads, kABlocks) cdm_accumulate_kernel(SEG
         return;
     const CdmCtl* c = S.ctl;
     const Dim3 D{S.w, S.h, S.d};
-    const unsigned pitch = (unsigned)S.ppitch, plane = pitch * (unsigned)D.h;
-    const int tiles = S.tnb / D.d, z = tile / tiles;
-    const unsigned p0 = (unsigned)(tile - z * tiles) * kTile + threadIdx.x;
-    const long long cs = S.pplane, z0 = (long long)z * plane;
+    const unsigned pitch = (unsigned)S.ppitch, total = (unsigned)S.pplane;
+    const unsigned p0 = (unsigned)tile * kTile + threadIdx.x;
+    const long long cs = S.pplane;
     // the update's loads go out before the loop flag is waited for
     float n0[kAVox], n1[kAVox], n2[kAVox];
 #pragma unroll
     for (int k = 0; k < kAVox; ++k) {
         const unsigned p = p0 + kAThreads * k;
-        const float* const q = S.aux_d + z0 + p;
-        n0[k] = load_now(q, p < plane);
-        n1[k] = load_now(q + cs, p < plane);
-        n2[k] = load_now(q + 2 * cs, p < plane);
+        const float* const q = S.aux_d + p;
+        n0[k] = load_now(q, p < total);
+        n1[k] = load_now(q + cs, p < total);
+        n2[k] = load_now(q + 2 * cs, p < total);
     }
     const int done = c->done, from = c->from;
     const float scale = c->scale;
@@ -1470,24 +1493,25 @@ __global__ void __launch_bounds__(kAThreads, kABlocks) cdm_accumulate_kernel(SEG
     if (S.ndim == 2 || !narrow(S)) {
         const Accumulate A{S.aux_d, cd, S.tmp_d, D, S.ndim, scale};
         for (unsigned p = p0; p < p0 - threadIdx.x + kTile; p += kAThreads) {
-            const int y = (int)(p / pitch), x = (int)(p - (unsigned)y * pitch);
-            const float* const q = A.nd + z0 + p;
-            if (p < plane && x < D.w)
-                accumulate_voxel(A, x, y, z, z0 + p, cs, 1, pitch, plane, q[0], q[cs], q[2 * cs]);
+            const Place at(p, pitch, D.h);
+            const float* const q = A.nd + p;
+            if (p < total && at.x < D.w)
+                accumulate_voxel(A, at.x, at.y, at.z, p, cs, 1, pitch, (long long)pitch * D.h, q[0], q[cs], q[2 * cs]);
         }
         return;
     }
     // below, offsets in bytes fit 32 bits and coordinates are exact floats
     const SampleGeo G{D.w, D.h, 0, (float)(D.w - 1), (float)(D.h - 1), (float)(D.d - 1)};
     const char* const base[3] = {(const char*)cd, (const char*)(cd + cs), (const char*)(cd + 2 * cs)};
-    int y = (int)(p0 / pitch), x = (int)(p0 - (unsigned)y * pitch);
+    const unsigned plane = pitch * (unsigned)D.h;
+    Place at(p0, pitch, D.h);
 #pragma unroll
     for (int k = 0; k < kAVox; ++k) {
         const unsigned p = p0 + kAThreads * k;
-        if (p < plane && x < D.w) {
+        if (p < total && at.x < D.w) {
             const float dx = n0[k] * scale, dy = n1[k] * scale, dz = n2[k] * scale;
-            const float X = u8_to_f(x), Y = u8_to_f(y), Z = u8_to_f(z), px = dx + X, py = dy + Y, pz = dz + Z;
-            float* const o = S.tmp_d + z0 + p;
+            const float X = u8_to_f(at.x), Y = u8_to_f(at.y), Z = u8_to_f(at.z), px = dx + X, py = dy + Y, pz = dz + Z;
+            float* const o = S.tmp_d + p;
             if (!(dx == 0.0f && dy == 0.0f && dz == 0.0f) && !(px < 0.0f || py < 0.0f || pz < 0.0f) && px < G.wl &&
                 py < G.hl && pz < G.dl) {
                 float f[3][2], r[8];
@@ -1506,14 +1530,13 @@ __global__ void __launch_bounds__(kAThreads, kABlocks) cdm_accumulate_kernel(SEG
                 o[cs] = a[1] - Y;
                 o[2 * cs] = a[2] - Z;
             } else {
-                o[0] = __ldg(cd + z0 + p);
-                o[cs] = __ldg(cd + z0 + p + cs);
-                o[2 * cs] = __ldg(cd + z0 + p + 2 * cs);
+                o[0] = __ldg(cd + p);
+                o[cs] = __ldg(cd + p + cs);
+                o[2 * cs] = __ldg(cd + p + 2 * cs);
             }
         }
         if (k + 1 < kAVox)
-            for (x += kAThreads; x >= (int)pitch; x -= (int)pitch)
-                ++y;
+            at.advance(kAThreads, pitch, D.h);
     }
 }
 
@@ -1576,15 +1599,14 @@ __global__ void __launch_bounds__(kTThreads) cdm_smooth_compose_kernel(SEG_ARGS)
     T* __restrict__ const Js = (T*)S.Js;
     const Dim3 D{S.w, S.h, S.d};
     const unsigned pitch = (unsigned)S.ppitch;
-    const int tiles = S.tnb / D.d, z = tile / tiles;
-    const unsigned tp = (unsigned)(tile - z * tiles) * kTile;  // the tile's first position in its plane
+    const unsigned tp = (unsigned)tile * kTile;  // the tile's first position
     const int lane = threadIdx.x & 31, warp = threadIdx.x & ~31;
     __shared__ float4 field[3][kTThreads];
     if ((pitch & 3) == 0) {
         const unsigned P = pitch / 4, plane = P * (unsigned)D.h, total = plane * (unsigned)D.d;
-        const unsigned q = tp / 4 + threadIdx.x, xq = q % P, i = (unsigned)z * plane + q;
+        const unsigned i = tp / 4 + threadIdx.x, xq = i % P;
         const int rem = D.w & 3;
-        const bool on = q < plane, row_end = xq == P - 1;
+        const bool on = i < total, row_end = xq == P - 1;
         const bool fix1 = row_end && rem == 1, fix2 = row_end && rem == 2, fix3 = row_end && rem == 3;
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
@@ -1605,7 +1627,7 @@ __global__ void __launch_bounds__(kTThreads) cdm_smooth_compose_kernel(SEG_ARGS)
                 float xl = __shfl_up_sync(0xffffffffu, tail, 1), xr = __shfl_down_sync(0xffffffffu, cur.x, 1);
                 if (lane == 0)
                     xl = one(4LL * i - 1 - (xq == 0 && rem ? 4 - rem : 0));
-                if (lane == 31 || q + 1 == plane)
+                if (lane == 31 || i + 1 == total)
                     xr = one(4LL * i + 4);
                 const float n1 = fix1 ? xr : cur.y, n2 = fix2 ? xr : cur.z, n3 = fix3 ? xr : cur.w;
                 r.x = cur.x * w_1 + ((((((0.0f + n1) + xl) + yb.x) + ya.x) + up.x) + down.x) * w_6;
@@ -1622,10 +1644,10 @@ __global__ void __launch_bounds__(kTThreads) cdm_smooth_compose_kernel(SEG_ARGS)
         for (int k = 0; k < 3; ++k)
             for (int j = 0; j < 4; ++j) {
                 const int v = 4 * warp + 32 * j + lane;
-                const long long p = (long long)tp + v, i = z * wh + p;
+                const long long i = (long long)tp + v;
                 const float* __restrict__ const d = S.tmp_d + k * S.pplane;
                 float* const out = dst + k * S.pplane;
-                if (p >= wh)
+                if (i >= n)
                     continue;
                 float r;
                 if (sm == 0.0f)
@@ -1649,19 +1671,19 @@ __global__ void __launch_bounds__(kTThreads) cdm_smooth_compose_kernel(SEG_ARGS)
     const bool fast = S.ndim != 2 && narrow(S);
     const SampleGeo G = sample_geo(D);
     const int v0 = 4 * warp + lane;
-    int y = (int)((tp + v0) / pitch), x = (int)(tp + v0 - (unsigned)y * pitch);
+    Place at(tp + v0, pitch, D.h);
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
         const int v = v0 + 32 * k;
         const float dx = reinterpret_cast<const float*>(field[0])[v], dy = reinterpret_cast<const float*>(field[1])[v],
                     dz = reinterpret_cast<const float*>(field[2])[v];
-        if (y < D.h && x < D.w) {
-            const int j = (z * D.h + y) * D.w + x;
-            Js[j] = fast ? compose_narrow(Is, G, (unsigned)j, x, y, z, dx, dy, dz)
-                         : compose_pixel(Is, D, S.ndim, j, x, y, z, dx, dy, dz);
+        if (at.z < D.d && at.x < D.w) {
+            const int j = (at.z * D.h + at.y) * D.w + at.x;
+            Js[j] = fast ? compose_narrow(Is, G, (unsigned)j, at.x, at.y, at.z, dx, dy, dz)
+                         : compose_pixel(Is, D, S.ndim, j, at.x, at.y, at.z, dx, dy, dz);
         }
-        for (x += 32; x >= (int)pitch; x -= (int)pitch)
-            ++y;
+        if (k < 3)
+            at.advance(32, pitch, D.h);
     }
 }
 
