@@ -41,7 +41,7 @@ DIMS = [(91, 109, 91), (182, 218, 182), (128, 128, 128), (68, 66, 70), (4, 4, 20
 def test_poisson_threads_have_work(shapes, dims):
     """The sweeps' threads have places for at most twice the padded voxels (four a place), but for
     a block a component; and padded rows take at most 60 % more than their voxels (5 of 8)."""
-    pitch, plane, _, pnb, pdz, _ = shapes("dims", *dims)
+    pitch, plane, _, pnb, pdz = shapes("dims", *dims)[:5]
     assert pnb * 256 * max(pdz, 1) <= 2 * 3 * (plane / 4) + 3 * 256 * max(pdz, 1)
     n = dims[0] * dims[1] * dims[2]
     assert plane <= 1.6 * n and pitch * dims[1] * dims[2] == plane
@@ -50,5 +50,17 @@ def test_poisson_threads_have_work(shapes, dims):
 @pytest.mark.parametrize("dims", DIMS)
 def test_tail_blocks_have_work(shapes, dims):
     """The tail launches have a block for each 512 places of a component."""
-    _, plane, _, _, _, tnb = shapes("dims", *dims)
+    plane, tnb = (shapes("dims", *dims)[k] for k in (1, 5))
     assert 512 * (tnb - 1) < plane <= 512 * tnb
+
+
+@pytest.mark.parametrize("dims", DIMS)
+def test_float_gradient_tiles_are_filled(shapes, dims):
+    """The float gradient's tiles are kept where a quarter of their voxels, at least, are the
+    volume's; ordinary grids keep them."""
+    each = shapes("dims", *dims)[6]
+    n = dims[0] * dims[1] * dims[2]
+    depth = 2 if n < 200000 else 4
+    tiles = -(-dims[0] // 32) * -(-dims[1] // 8) * -(-dims[2] // depth)
+    assert each or 4 * n > tiles * 32 * 8 * depth
+    assert not (each and min(dims) >= 36)

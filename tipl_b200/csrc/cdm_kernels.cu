@@ -652,6 +652,59 @@ __device__ __forceinline__ double gradient_r_f32(const CdmSeg& S, int blk, int m
     return csum;
 }
 
+// The same a voxel a thread, from global memory: for the volumes of cdm_gradient_each.
+__device__ __forceinline__ double gradient_r_f32_each(const CdmSeg& S, int blk, int mod)
+{
+    const Dim3 D{S.w, S.h, S.d};
+    const float* __restrict__ Js = (const float*)S.Js;
+    const float* __restrict__ It = (const float*)S.It[mod];
+    float* __restrict__ nd = S.new_d;
+    const long long n = D.n(), w = D.w, wh = D.wh();
+    double csum = 0.0;
+    for (long long i = blk * (long long)kFThreads + threadIdx.x; i < n; i += (long long)S.nblk * kFThreads) {
+        int x, y, z;
+        unflat((int)i, D, x, y, z);
+        float3 out = make_float3(0.0f, 0.0f, 0.0f);
+        const float js = Js[i], it = It[i];
+        if (!(js == 0.0f || it == 0.0f)) {
+            const int xu = min(D.w - x - 1, 2), yu = min(D.h - y - 1, 2), zu = min(D.d - z - 1, 2);
+            const int xl = min(x, 2), yl = min(y, 2), zl = min(z, 2);
+            double sx = 0.0, sy = 0.0, sxx = 0.0, syy = 0.0, sxy = 0.0;
+            auto add = [&](long long k) {
+                const float j = Js[k], t = It[k];
+                const double dj = j, dt = t;
+                sx += dj;
+                sy += dt;
+                sxx = __fma_rn(dj, dj, sxx);
+                syy = __fma_rn(dt, dt, syy);
+                sxy += (double)__fmul_rn(j, t);
+            };
+            for (int a = 0; a <= zu + zl; ++a) {  // offsets 0, 1, 2, -1, -2 where they are inside
+                const long long zi = i + (a <= zu ? a : zu - a) * wh;
+                for (int b = 0; b <= yu + yl; ++b) {
+                    const long long yi = zi + (b <= yu ? b : yu - b) * w;
+                    for (int c = 0; c <= xu; ++c)
+                        add(yi + c);
+                    for (int c = 1; c <= xl; ++c)
+                        add(yi - c);
+                }
+            }
+            Reg r;
+            regress_finish(sx, sy, sxx, syy, sxy, (xu + xl + 1) * (yu + yl + 1) * (zu + zl + 1), r);
+            if (r.a > 0.0f) {
+                const float3 g = grad_at(Js, D, x, y, z, i);
+                const float s = r.r2 * (js * r.a + r.b - it);
+                out.x = 0.0f + g.x * s;
+                out.y = 0.0f + g.y * s;
+                out.z = 0.0f + g.z * s;
+                csum += (double)-r.r2;
+            }
+        }
+        store_term(nd + update_index(S, i), update_comp(S), out, mod);
+    }
+    return csum;
+}
+
 template <bool MULTI>
 __global__ void __launch_bounds__(kFThreads, 3) cdm_gradient_r_f32_kernel(SEG_ARGS,
                                                                           int mod)
@@ -667,9 +720,26 @@ __global__ void __launch_bounds__(kFThreads, 3) cdm_gradient_r_f32_kernel(SEG_AR
     // there are not enough tiles of four to fill the chip (91x109x91: 71.0 us with two, 65.6
     // with four; 64^3: 32.0 / 30.1; 46x55x46: 25.3 / 27.4; 23x28x23: 14.8 / 20.6).
     const long long n = (long long)S.w * S.h * S.d;
-    const double cs = n < 200000 ? gradient_r_f32<2>(S, blk, mod, smem) : gradient_r_f32<4>(S, blk, mod, smem);
+    const double cs = MULTI && S.each ? gradient_r_f32_each(S, blk, mod)
+                      : n < 200000    ? gradient_r_f32<2>(S, blk, mod, smem)
+                                      : gradient_r_f32<4>(S, blk, mod, smem);
     __shared__ double red[32];
     const double csum = block_sum(cs, red);
+    if (threadIdx.x == 0)
+        S.cost_part[blk] = csum;
+    if (last_block_of_segment(S))
+        control_block(S, mod);
+}
+
+// One level of that form: 64 registers, four blocks an SM instead of the three of the tiles.
+__global__ void __launch_bounds__(kFThreads) cdm_gradient_r_f32_each_kernel(SEG_ARGS, int mod)
+{
+    const CdmSeg& S = one;
+    const int blk = (int)blockIdx.x;
+    if (S.ctl->done || mod >= max(S.nmod, 1))
+        return;
+    __shared__ double red[32];
+    const double csum = block_sum(gradient_r_f32_each(S, blk, mod), red);
     if (threadIdx.x == 0)
         S.cost_part[blk] = csum;
     if (last_block_of_segment(S))
@@ -890,6 +960,24 @@ void cdm_set_walk(CdmSeg* s, int n)
     }
 }
 
+// Whether the float 'r' gradient takes a voxel a thread: for volumes of few voxels on an axis,
+// which fill little of a tile and have few of the window's taps inside.  The lower of two
+// estimates in us: each voxel its taps, against the tiles, of which small levels have more than
+// blocks.  Launches in tiles / so: 1x300x300 290 / 15.7 us, 3x300x300 202 / 59, 7x300x300 203 /
+// 119, 1024x1024x1 168 / 60, 300x2x300 51 / 26, 8x60x60 32 / 21; and where tiles are kept:
+// 9x300x300 206 / 187, 300x300x3 36 / 47, 33x33x33 21 / 23, 91x109x91 80 / 183.
+static int gradient_each(int w, int h, int d)
+{
+    auto taps = [](int n) { return n < 4 ? n : 5.0 - 6.0 / n; };  // inside, on average
+    const long long n = (long long)w * h * d;
+    const int v = n < 200000 ? 2 : 4;
+    const long long tiles = (long long)((w + kFX - 1) / kFX) * ((h + kFY - 1) / kFY) * ((d + v - 1) / v);
+    const double t = taps(w) * taps(h) * taps(d);
+    const int blocks = cdm_blocks_for(n);
+    const double each = std::max(9.0 + 0.09 * t, 2.1e-6 * (double)n * (t + 14.0));
+    return each < (v == 2 ? 7.0 + 7.2 * (double)((tiles + blocks - 1) / blocks) : 0.06 * (double)tiles);
+}
+
 // Launch shapes that follow from a level's dims alone.
 void cdm_set_dims(CdmSeg& s, int w, int h, int d)
 {
@@ -907,6 +995,7 @@ void cdm_set_dims(CdmSeg& s, int w, int h, int d)
     s.ppitch = pad ? padded : w;
     s.pplane = s.ppitch * rows;
     cdm_set_walk(&s, 1);
+    s.each = gradient_each(w, h, d);
     s.tnb = (int)((s.pplane + kTile - 1) / kTile);
 }
 
@@ -1919,7 +2008,9 @@ cudaError_t launch_cdm_gradient(const CdmSegs& L, int pix, int gradient_type,
         }
         SEG_LAUNCH(cdm_gradient_box_u8_kernel<true>, cdm_gradient_box_u8_kernel<false>, kUThreads,
                    box_smem<8>(), mod);
-    } else if (gradient_type == 'r')
+    } else if (gradient_type == 'r' && L.n == 1 && L.host->each)
+        cdm_gradient_r_f32_each_kernel<<<L.blocks, kFThreads, 0, st>>>(L.dev, L.n, *L.host, mod);
+    else if (gradient_type == 'r')
         SEG_LAUNCH(cdm_gradient_r_f32_kernel<true>, cdm_gradient_r_f32_kernel<false>, kFThreads, 0, mod);
     else if (pix == 0)
         SEG_LAUNCH((cdm_gradient_d_kernel<uint8_t, true>), (cdm_gradient_d_kernel<uint8_t, false>), kCdmThreads, 0, mod);

@@ -102,6 +102,7 @@ struct CdmSeg {
     // planar: the fields (field, new_d, aux_d, tmp_d) are held as component planes of pplane
     // floats, rows ppitch apart, as the Poisson launches take them; else interleaved xyz
     int planar;
+    int each;  // the float 'r' gradient takes a voxel a thread, not tiles
     long long ppitch, pplane;
     long long planes_floats() const { return 3 * pplane; }
 };
