@@ -4,7 +4,7 @@
 //   cdm_shapes probe <call>           the n-th runtime call of the cluster check fails (0: none);
 //                                     prints whether clusters are used, and the error left behind
 //   cdm_shapes dims <w> <h> <d>       a level's layout and launch shapes: ppitch pplane nblk pnb
-//                                     pdz tnb each
+//                                     pdz tnb each shallow
 #include <atomic>
 #include <cstdio>
 #include <cstdlib>
@@ -73,7 +73,8 @@ int main(int argc, char** argv)
     if (argc == 5 && !std::strcmp(argv[1], "dims")) {
         regb::CdmSeg s{};
         regb::cdm_set_dims(s, std::atoi(argv[2]), std::atoi(argv[3]), std::atoi(argv[4]));
-        std::printf("%lld %lld %d %d %d %d %d\n", s.ppitch, s.pplane, s.nblk, s.pnb, s.pdz, s.tnb, s.each);
+        std::printf("%lld %lld %d %d %d %d %d %d\n", s.ppitch, s.pplane, s.nblk, s.pnb, s.pdz, s.tnb, s.each,
+                    s.shallow);
         return 0;
     }
     return 2;

@@ -64,3 +64,14 @@ def test_float_gradient_tiles_are_filled(shapes, dims):
     tiles = -(-dims[0] // 32) * -(-dims[1] // 8) * -(-dims[2] // depth)
     assert each or 4 * n > tiles * 32 * 8 * depth
     assert not (each and min(dims) >= 36)
+
+
+@pytest.mark.parametrize("dims", DIMS + [(300, 1, 300), (300, 2, 300), (23, 28, 23), (46, 55, 46)])
+def test_uint8_gradient_tile_depth(shapes, dims):
+    """The uint8 gradient's tiles are no deeper than the volume needs, and those of 2 planes are
+    few enough for the blocks that share them."""
+    nblk, shallow = (shapes("dims", *dims)[k] for k in (2, 7))
+    tiles = -(-dims[0] // 32) * -(-dims[1] // 8) * -(-dims[2] // 2)
+    assert shallow or dims[2] > 2
+    assert not shallow or dims[2] <= 2 or tiles <= 3 * min(nblk, 444)
+    assert shallow == 1 if dims in ((23, 28, 23), (46, 55, 46)) else True

@@ -482,10 +482,7 @@ __global__ void __launch_bounds__(kUThreads) cdm_gradient_box_u8_kernel(SEG_ARGS
     if (S.ctl->done || mod >= max(S.nmod, 1))
         return;
     extern __shared__ __align__(16) unsigned char smraw[];
-    // Tiles of 2 planes where tiles of 8 would leave most SMs idle (23x28x23: 9.8 us / 14.0;
-    // 64^3: 20.4 / 18.6)
-    const long long n = (long long)S.w * S.h * S.d;
-    const double cs = n < 200000 ? gradient_box_u8<2>(S, blk, mod, smraw) : gradient_box_u8<8>(S, blk, mod, smraw);
+    const double cs = S.shallow ? gradient_box_u8<2>(S, blk, mod, smraw) : gradient_box_u8<8>(S, blk, mod, smraw);
     __shared__ double red[32];
     const double csum = block_sum(cs, red);
     if (threadIdx.x == 0)
@@ -978,6 +975,17 @@ static int gradient_each(int w, int h, int d)
     return each < (v == 2 ? 7.0 + 7.2 * (double)((tiles + blocks - 1) / blocks) : 0.06 * (double)tiles);
 }
 
+// Whether the uint8 'r' gradient's tiles are 2 planes deep, not 8: where there are no more planes
+// (1024x1024x1 63 / 89 us), and on levels whose tiles of 8 would leave most SMs idle (23x28x23
+// 9.8 / 14.0; 64^3 20.1 / 19.6), unless a block has several of them in turn (short rows or
+// columns: 300x2x300 35.5 / 28.8).
+static int gradient_shallow(int w, int h, int d)
+{
+    const long long n = (long long)w * h * d;
+    const long long tiles = (long long)((w + kUX - 1) / kUX) * ((h + kUY - 1) / kUY) * ((d + 1) / 2);
+    return d <= 2 || (n < 200000 && tiles <= 3 * std::min(cdm_blocks_for(n), 148 * 3));
+}
+
 // Launch shapes that follow from a level's dims alone.
 void cdm_set_dims(CdmSeg& s, int w, int h, int d)
 {
@@ -996,6 +1004,7 @@ void cdm_set_dims(CdmSeg& s, int w, int h, int d)
     s.pplane = s.ppitch * rows;
     cdm_set_walk(&s, 1);
     s.each = gradient_each(w, h, d);
+    s.shallow = gradient_shallow(w, h, d);
     s.tnb = (int)((s.pplane + kTile - 1) / kTile);
 }
 

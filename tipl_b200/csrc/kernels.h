@@ -102,7 +102,8 @@ struct CdmSeg {
     // planar: the fields (field, new_d, aux_d, tmp_d) are held as component planes of pplane
     // floats, rows ppitch apart, as the Poisson launches take them; else interleaved xyz
     int planar;
-    int each;  // the float 'r' gradient takes a voxel a thread, not tiles
+    int each;     // the float 'r' gradient takes a voxel a thread, not tiles
+    int shallow;  // the uint8 'r' gradient's tiles are 2 planes deep, not 8
     long long ppitch, pplane;
     long long planes_floats() const { return 3 * pplane; }
 };
