@@ -158,7 +158,10 @@ __device__ __forceinline__ T compose_narrow(const T* __restrict__ Is, const Samp
     return assign_pix<T>(acc);
 }
 
-template <typename T, bool MULTI>
+// PLANAR: the field's layout, known here to keep its index arithmetic out of the loop, as the
+// dimension is (interleaved, 2048x2048x1: 24.5 us with both looked up for each voxel, 18.7 so;
+// 256x256x200 127 / 119).
+template <typename T, bool MULTI, bool PLANAR>
 __global__ void __launch_bounds__(kCdmThreads) cdm_compose_kernel(SEG_ARGS, int mod)
 {
     SEG_BEGIN
@@ -167,14 +170,21 @@ __global__ void __launch_bounds__(kCdmThreads) cdm_compose_kernel(SEG_ARGS, int 
     const T* __restrict__ Is = (const T*)S.Is[mod];
     T* __restrict__ Js = (T*)S.Js;
     const float* __restrict__ f = S.field[S.ctl->cur];
-    const long long cs = update_comp(S);
-    for (long long i = first; i < n; i += stride) {
-        const long long o = update_index(S, i);
-        const float dx = f[o], dy = f[o + cs], dz = f[o + 2 * cs];
-        int x, y, z;
-        unflat((int)i, D, x, y, z);
-        Js[i] = compose_pixel(Is, D, S.ndim, (int)i, x, y, z, dx, dy, dz);
-    }
+    const long long cs = PLANAR ? S.pplane : 1;
+    auto pixels = [&](int ndim) {
+        for (long long i = first; i < n; i += stride) {
+            const long long o = PLANAR ? update_index(S, i) : 3 * i;
+            const float dx = f[o], dy = f[o + cs], dz = ndim == 2 ? 0.0f : f[o + 2 * cs];
+            int x = 0, y = 0, z = 0;
+            if (dx != 0.0f || dy != 0.0f || dz != 0.0f)
+                unflat((int)i, D, x, y, z);
+            Js[i] = compose_pixel(Is, D, ndim, (int)i, x, y, z, dx, dy, dz);
+        }
+    };
+    if (S.ndim == 2)
+        pixels(2);
+    else
+        pixels(3);
 }
 
 __device__ void control_block(const CdmSeg& S, int mod);
@@ -1985,10 +1995,18 @@ cudaError_t launch_cdm_compose(const CdmSegs& L, int pix, cudaStream_t st, int m
 {
     if (mod < 0 || mod >= kCdmMaxModalities)
         return cudaErrorInvalidValue;
-    if (pix == 0)
-        SEG_LAUNCH((cdm_compose_kernel<uint8_t, true>), (cdm_compose_kernel<uint8_t, false>), kCdmThreads, 0, mod);
-    else
-        SEG_LAUNCH((cdm_compose_kernel<float, true>), (cdm_compose_kernel<float, false>), kCdmThreads, 0, mod);
+    if (L.host->planar) {
+        if (pix == 0)
+            SEG_LAUNCH((cdm_compose_kernel<uint8_t, true, true>), (cdm_compose_kernel<uint8_t, false, true>), kCdmThreads,
+                       0, mod);
+        else
+            SEG_LAUNCH((cdm_compose_kernel<float, true, true>), (cdm_compose_kernel<float, false, true>), kCdmThreads, 0,
+                       mod);
+    } else if (L.n == 1) {
+        auto kernel = pix ? cdm_compose_kernel<float, false, false> : cdm_compose_kernel<uint8_t, false, false>;
+        kernel<<<L.blocks, kCdmThreads, 0, st>>>(L.dev, L.n, *L.host, mod);
+    } else
+        return cudaErrorInvalidValue;
     count_launch();
     return cudaGetLastError();
 }
