@@ -1043,17 +1043,18 @@ __device__ __forceinline__ float load_now(const float* __restrict__ p, bool ok)
     return f;
 }
 
-// One block's part of a sweep: float4 column q of the `span` that its threads' columns are taken
-// from (a plane, or the whole component for planes [0, 1)), planes [z0, z1).  FIRST: the input is
-// the right-hand side times c6.  EDGE: some tap of the block may lie outside the field.
-template <bool FIRST, bool EDGE>
+// One block's part of a sweep: float4 column q of a plane, planes [z0, z1).  FIRST: the input
+// is the right-hand side times c6.  EDGE: some tap of the block may lie outside the field.  WHOLE:
+// float4 q of the component instead, for planes [0, 1).
+template <bool FIRST, bool EDGE, bool WHOLE = false>
 __device__ __forceinline__ void poisson_walk(const CdmSeg& S, const float4* __restrict__ in, const float4* __restrict__ rhs,
-                                             float4* __restrict__ out, unsigned q, unsigned span, int z0, int z1, int done)
+                                             float4* __restrict__ out, unsigned q, int z0, int z1, int done)
 {
     const unsigned P = (unsigned)(S.ppitch / 4), plane = P * (unsigned)S.h, total = plane * (unsigned)S.d;
     const float c6 = poisson_weight(S);
     const int rem = S.w & 3, lane = threadIdx.x & 31;
     const unsigned xq = q % P;
+    const unsigned span = WHOLE ? total : plane;
     const bool on = q < span, row_end = xq == P - 1;
     const bool fix1 = row_end && rem == 1, fix2 = row_end && rem == 2, fix3 = row_end && rem == 3;
     unsigned i = (unsigned)z0 * plane + q;
@@ -1152,22 +1153,21 @@ __global__ void __launch_bounds__(kPThreads, 4) cdm_poisson_kernel(SEG_ARGS, int
         if (!done)
             poisson_flat<FIRST>(S, in, rhs, out, t, per);
     } else {
-        const unsigned plane = (unsigned)(S.ppitch / 4) * (unsigned)S.h;
         const float4* const in4 = reinterpret_cast<const float4*>(in);
         const float4* const rhs4 = reinterpret_cast<const float4*>(rhs);
         float4* const out4 = reinterpret_cast<float4*>(out);
         if (S.pdz == 0) {
             const unsigned q = (unsigned)t * kPThreads + threadIdx.x;
-            poisson_walk<FIRST, true>(S, in4, rhs4, out4, q, plane * (unsigned)S.d, 0, 1, done);
+            poisson_walk<FIRST, true, true>(S, in4, rhs4, out4, q, 0, 1, done);
             return;
         }
         const int nz = (S.d + S.pdz - 1) / S.pdz, nq = per / nz;
         const int z0 = t / nq * S.pdz, z1 = min(S.d, z0 + S.pdz);
         const unsigned q = (unsigned)(t % nq) * kPThreads + threadIdx.x;
         if (z0 == 0 || z1 == S.d)  // (a plane below and above covers the rows and voxels beside)
-            poisson_walk<FIRST, true>(S, in4, rhs4, out4, q, plane, z0, z1, done);
+            poisson_walk<FIRST, true>(S, in4, rhs4, out4, q, z0, z1, done);
         else
-            poisson_walk<FIRST, false>(S, in4, rhs4, out4, q, plane, z0, z1, done);
+            poisson_walk<FIRST, false>(S, in4, rhs4, out4, q, z0, z1, done);
     }
 }
 
