@@ -1,4 +1,4 @@
-"""The Gaussian where the number of planes a warp walks changes (3, 6, 9, 15), with depths that end
+"""The Gaussian where the number of planes a warp walks changes (3, 6, 15), with depths that end
 within a turn of three planes -- against the oracle, bit for bit."""
 import numpy as np
 import pytest
@@ -7,9 +7,9 @@ import tipl_b200 as tb
 
 pytestmark = pytest.mark.gpu
 
-# 1 to 8 column blocks a plane: at most 444 blocks with 3, 6 and 9 planes, and more with 9
-SHAPES = [(1332, 16, 32), (1333, 16, 32), (2665, 15, 30), (3997, 16, 20), (166, 33, 63), (167, 60, 60), (334, 60, 50),
-          (500, 60, 50)]
+# 1 to 8 column blocks a plane: at most and more than 444 blocks with 3 planes, and 592 with 6
+SHAPES = [(1332, 16, 32), (1333, 16, 32), (3552, 15, 30), (3553, 16, 20), (166, 33, 63), (167, 60, 60), (444, 60, 50),
+          (445, 60, 50)]
 
 
 @pytest.mark.parametrize("shape", SHAPES)

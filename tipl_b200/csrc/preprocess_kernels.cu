@@ -16,7 +16,7 @@ namespace {
 
 // ------------------------------------------------------------------ Gaussian
 // One round of the reference's x, y, z passes fused in one kernel, from any storage type.  A
-// warp owns 32 columns of four rows and walks up to kGz planes: a plane's six rows (a halo row
+// warp owns 32 columns of four rows and walks WALK planes: a plane's six rows (a halo row
 // on either side) are loaded one plane ahead, x neighbours come by shuffles (the two columns
 // beside the tile from lanes 0 and 31), the y pass adds rows of the thread's registers, and
 // the z pass the last three planes.  Halo and edge samples come from clamped coordinates,
@@ -28,7 +28,7 @@ namespace {
 // 256x256x200 with smallest and largest value: 92 us as a widening pass, a shared-memory tile
 // with three barriers and a pass for the extremes, 34 so; two planes ahead or rows by six or
 // eight gave no more (48, 38, 33).
-constexpr int kGx = 32, kGRows = 4, kGWarps = 4, kGz = 15, kGThreads = 32 * kGWarps;
+constexpr int kGx = 32, kGRows = 4, kGWarps = 4, kGThreads = 32 * kGWarps;
 
 __device__ __forceinline__ float tap3(float l, float c, float r)
 {
@@ -36,15 +36,15 @@ __device__ __forceinline__ float tap3(float l, float c, float r)
     return __fadd_rn(__fadd_rn(l, __fadd_rn(c, c)), r);
 }
 
-template <int DT>
+template <int DT, int WALK>
 __global__ void __launch_bounds__(kGThreads) gaussian_round_kernel(const void* __restrict__ in,
                                                                    float* __restrict__ out, int w, int h, int d,
-                                                                   float scale, int apply_scale, int walk,
+                                                                   float scale, int apply_scale,
                                                                    unsigned* __restrict__ mm)
 {
     constexpr int kRows = kGRows + 2;
     const int lane = threadIdx.x & 31;
-    const int x0 = blockIdx.x * kGx, y0 = (blockIdx.y * kGWarps + (threadIdx.x >> 5)) * kGRows, z0 = blockIdx.z * walk;
+    const int x0 = blockIdx.x * kGx, y0 = (blockIdx.y * kGWarps + (threadIdx.x >> 5)) * kGRows, z0 = blockIdx.z * WALK;
     if (y0 >= h)
         return;
     const int x = x0 + lane, xc = min(x, w - 1), xh = lane == 0 ? max(x0 - 1, 0) : min(x0 + kGx, w - 1);
@@ -84,8 +84,8 @@ __global__ void __launch_bounds__(kGThreads) gaussian_round_kernel(const void* _
     pass(ring[1]);
     load(z0 + 1);
     // by threes, so that the ring of planes stays in registers
-    static_assert(kGz % 3 == 0, "whole turns");
-    for (int k0 = 0; k0 < walk; k0 += 3) {
+    static_assert(WALK % 3 == 0, "whole turns");
+    for (int k0 = 0; k0 < WALK; k0 += 3) {
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
             const int z = z0 + k0 + j;
@@ -397,17 +397,21 @@ __global__ void __launch_bounds__(kPThreads) otsu_normalize_kernel(const float* 
         out[t] = (uint8_t)value(v[t]);
 }
 
-// Planes a warp of the Gaussian walks: the fewest (whole turns of the ring) with no more blocks
-// than three an SM, so that small volumes are not a chain of planes on a few SMs.  With 3 / 6 /
-// 15 planes: 16^3 to 64^3 3.1 / 4.0 / 6.7 us, 100^3 6.4 / 6.2 / 8.0, 160^3 14.0 / 12.0 / 11.9,
-// 182x218x182 24.9 / 21.1 / 19.3.
-int gaussian_walk(int w, int h, int d)
+// A launch with WALK planes a warp.
+template <int WALK>
+cudaError_t gaussian_launch(const void* in, int dtype, float* out, int w, int h, int d, float scale, int apply_scale,
+                            unsigned* mm, cudaStream_t st)
 {
-    const long long columns = (long long)((w + kGx - 1) / kGx) * ((h + kGRows * kGWarps - 1) / (kGRows * kGWarps));
-    for (int walk : {3, 6, 9})
-        if (columns * ((d + walk - 1) / walk) <= 148 * 3)
-            return walk;
-    return kGz;
+    const int rows = kGRows * kGWarps;
+    const dim3 grid((w + kGx - 1) / kGx, (h + rows - 1) / rows, (d + WALK - 1) / WALK);
+    switch (dtype) {
+    case 0: gaussian_round_kernel<0, WALK><<<grid, kGThreads, 0, st>>>(in, out, w, h, d, scale, apply_scale, mm); break;
+    case 1: gaussian_round_kernel<1, WALK><<<grid, kGThreads, 0, st>>>(in, out, w, h, d, scale, apply_scale, mm); break;
+    case 2: gaussian_round_kernel<2, WALK><<<grid, kGThreads, 0, st>>>(in, out, w, h, d, scale, apply_scale, mm); break;
+    case 3: gaussian_round_kernel<3, WALK><<<grid, kGThreads, 0, st>>>(in, out, w, h, d, scale, apply_scale, mm); break;
+    default: return cudaErrorInvalidValue;
+    }
+    return cudaGetLastError();
 }
 
 int pgrid(long long n)
@@ -417,20 +421,18 @@ int pgrid(long long n)
 
 }  // namespace
 
+// Small volumes walk fewer planes, so that a launch is not a chain of 15 on a few SMs: 3 while
+// that makes no more than three blocks an SM, 6 while no more than four.  With 3 / 6 / 15 planes:
+// 16^3 to 64^3 3.1 / 4.0 / 6.7 us, 100^3 6.4 / 6.2 / 8.0, 160^3 14.0 / 12.0 / 11.9, 182x218x182
+// 24.9 / 21.1 / 19.1.
 cudaError_t launch_gaussian_round(const void* in, int dtype, float* out, int w, int h, int d, float scale,
                                   int apply_scale, unsigned* mm, cudaStream_t st)
 {
-    const int rows = kGRows * kGWarps;
-    const int walk = gaussian_walk(w, h, d);
-    const dim3 grid((w + kGx - 1) / kGx, (h + rows - 1) / rows, (d + walk - 1) / walk);
-    switch (dtype) {
-    case 0: gaussian_round_kernel<0><<<grid, kGThreads, 0, st>>>(in, out, w, h, d, scale, apply_scale, walk, mm); break;
-    case 1: gaussian_round_kernel<1><<<grid, kGThreads, 0, st>>>(in, out, w, h, d, scale, apply_scale, walk, mm); break;
-    case 2: gaussian_round_kernel<2><<<grid, kGThreads, 0, st>>>(in, out, w, h, d, scale, apply_scale, walk, mm); break;
-    case 3: gaussian_round_kernel<3><<<grid, kGThreads, 0, st>>>(in, out, w, h, d, scale, apply_scale, walk, mm); break;
-    default: return cudaErrorInvalidValue;
-    }
-    return cudaGetLastError();
+    const long long columns = (long long)((w + kGx - 1) / kGx) * ((h + kGRows * kGWarps - 1) / (kGRows * kGWarps));
+    auto launch = columns * ((d + 2) / 3) <= 148 * 3   ? gaussian_launch<3>
+                  : columns * ((d + 5) / 6) <= 148 * 4 ? gaussian_launch<6>
+                                                       : gaussian_launch<15>;
+    return launch(in, dtype, out, w, h, d, scale, apply_scale, mm, st);
 }
 
 cudaError_t launch_otsu_hist(const float* v, long long n, const unsigned* mm, unsigned* hist, cudaStream_t st)
