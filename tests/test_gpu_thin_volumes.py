@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 # without padding; one plane; planes that use 77, 78, 80 and 95 % of the threads that walk them
 POISSON = [(300, 1, 1), (70, 1, 2), (66, 3, 2), (65, 40, 1), (70, 2, 3), (90, 4, 4), (67, 5, 6), (66, 7, 30), (70, 1, 37),
            (1, 1, 5000), (1, 1100, 1), (1, 1030, 2), (1, 1100, 5), (3, 1030, 2), (66, 28, 28), (66, 40, 40), (66, 41, 20),
-           (66, 44, 44), (70, 16, 16), (200, 8, 64)]
+           (66, 44, 44), (70, 16, 16), (200, 8, 64), (3000, 1, 2), (900, 7, 1), (1500, 3, 2), (70, 600, 2)]
 
 
 @pytest.mark.parametrize("shape", POISSON)

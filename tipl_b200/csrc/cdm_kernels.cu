@@ -913,7 +913,7 @@ __device__ __forceinline__ bool last_block_of_segment(const CdmSeg& S)
 // scalar loads each, the neighbouring rows and planes from L2), and so: 91x109x91 11.4 / 6.5 us,
 // 128^3 22.7 / 10.7, 182x218x182 103 / 53.  Levels of up to 64 planes of 1024 columns take the
 // clusters below instead (46x55x46, 12 sweeps: 49 / 40 / 17.6).
-constexpr int kPThreads = 256;
+constexpr int kPThreads = 256, kFlat = 4;
 constexpr int kPSweeps = 12;  // reg/cdm.hpp:165
 static_assert(kPSweeps % 2 == 0, "the result lands in aux_d");
 // The tail launches (accumulate, smooth and compose): a block takes kTile positions of a
@@ -947,8 +947,8 @@ void cdm_set_walk(CdmSeg* s, int n)
         return (e.ppitch & 3) || e.d == 1 || 5 * cols < 4 * blocks_of(cols) * kPThreads;
     };
     auto blocks = [&](const CdmSeg& e, int dz) {
-        if (e.ppitch & 3)  // four floats a thread (2x200000x1: 74 us, one a thread 114)
-            return 3 * blocks_of((e.pplane + 3) / 4);
+        if (e.ppitch & 3)
+            return 3 * blocks_of((e.pplane + kFlat - 1) / kFlat);
         return 3 * (whole(e) ? blocks_of(e.pplane / 4) : blocks_of(e.ppitch / 4 * e.h) * ((e.d + dz - 1) / dz));
     };
     int walk = 8;
@@ -1005,8 +1005,8 @@ void cdm_set_dims(CdmSeg& s, int w, int h, int d)
     s.nblk = cdm_blocks_for((long long)w * h * d);
     // component planes of the fields: rows padded to 4 voxels, unless that doubles them (rows of
     // one or two voxels; not where the sweeps then run in clusters) or costs memory that counts
-    // (other short rows of a huge volume).  12 sweeps with padded rows / so: 1x200000x1 86 / 48
-    // us, 2x200000x1 86 / 74, 2x300x300 50 / 48, but 3x300x300 50 / 64.
+    // (other short rows of a huge volume).  12 sweeps with padded rows / so: 1x200000x1 86 / 44
+    // us, 2x200000x1 86 / 74, 2x300x300 50 / 42; 9x1280x1200 1449 / 1600.
     const long long rows = (long long)h * d, padded = (w + 3LL) / 4 * 4;
     const bool pad = 4 * padded <= 5LL * w || cluster_holds(padded, h, d) ||
                      (padded < 2LL * w && padded * rows < (1LL << 24));
@@ -1113,15 +1113,41 @@ __device__ __forceinline__ void poisson_walk(const CdmSeg& S, const float4* __re
     }
 }
 
-// The part of block b in a sweep over unpadded rows: a float a thread.
+// The part of block b in a sweep over unpadded rows: kFlat runs of a float a thread, whose taps
+// are all on their way before the first is used (12 sweeps of 2x2000x5000: 3247 us a float after
+// the other, 2281 so; 9x1280x1200 2350 / 1600; 2x300x300 48 / 42).
 template <bool FIRST>
-__device__ void poisson_flat(const CdmSeg& S, const float* __restrict__ in, const float* __restrict__ rhs,
-                             float* __restrict__ out, long long b, long long blocks)
+__device__ __forceinline__ void poisson_flat(const CdmSeg& S, const float* __restrict__ in, const float* __restrict__ rhs,
+                                             float* __restrict__ out, unsigned b)
 {
-    const long long w = S.w, wh = w * S.h, n = wh * S.d;
+    const unsigned w = (unsigned)S.w, wh = w * (unsigned)S.h, n = wh * (unsigned)S.d;
     const float c6 = poisson_weight(S);
-    auto at = [&](long long k) { return FIRST ? __ldg(in + k) * c6 : __ldg(in + k); };
-    for (long long p = b * kPThreads + threadIdx.x; p < n; p += blocks * kPThreads) {
+    auto at = [&](unsigned k) { return FIRST ? __ldg(in + k) * c6 : __ldg(in + k); };
+    const unsigned first = b * (kFlat * kPThreads), p0 = first + threadIdx.x;
+    if (first >= wh && first + kFlat * kPThreads + wh <= n) {  // every tap is inside
+        float t[kFlat][7];
+#pragma unroll
+        for (int k = 0; k < kFlat; ++k) {
+            const unsigned p = p0 + k * kPThreads, i[6] = {p - 1, p + 1, p - w, p + w, p - wh, p + wh};
+            t[k][6] = __ldg(rhs + p);
+#pragma unroll
+            for (int j = 0; j < 6; ++j)
+                t[k][j] = at(i[j]);
+        }
+#pragma unroll
+        for (int k = 0; k < kFlat; ++k) {
+            float acc = t[k][6];
+#pragma unroll
+            for (int j = 0; j < 6; ++j)
+                acc -= t[k][j];
+            out[p0 + k * kPThreads] = acc * c6;
+        }
+        return;
+    }
+    for (int k = 0; k < kFlat; ++k) {
+        const unsigned p = p0 + k * kPThreads;
+        if (p >= n)
+            return;
         float acc = __ldg(rhs + p);
         if (p >= 1) acc -= at(p - 1);
         if (p < n - 1) acc -= at(p + 1);
@@ -1149,9 +1175,9 @@ __global__ void __launch_bounds__(kPThreads, 4) cdm_poisson_kernel(SEG_ARGS, int
     const float* const rhs = S.new_d + comp * S.pplane;
     const float* const in = FIRST ? rhs : (parity ? S.tmp_d : S.aux_d) + comp * S.pplane;
     float* const out = (FIRST || !parity ? S.tmp_d : S.aux_d) + comp * S.pplane;
-    if (S.ppitch & 3) {
+    if (MULTI && (S.ppitch & 3)) {
         if (!done)
-            poisson_flat<FIRST>(S, in, rhs, out, t, per);
+            poisson_flat<FIRST>(S, in, rhs, out, (unsigned)t);
     } else {
         const float4* const in4 = reinterpret_cast<const float4*>(in);
         const float4* const rhs4 = reinterpret_cast<const float4*>(rhs);
@@ -1169,6 +1195,20 @@ __global__ void __launch_bounds__(kPThreads, 4) cdm_poisson_kernel(SEG_ARGS, int
         else
             poisson_walk<FIRST, false>(S, in4, rhs4, out4, q, z0, z1, done);
     }
+}
+
+// One level of unpadded rows.
+template <bool FIRST>
+__global__ void __launch_bounds__(kPThreads, 4) cdm_poisson_flat_kernel(SEG_ARGS, int parity)
+{
+    const CdmSeg& S = one;
+    const int done = S.ctl->done;
+    const int per = S.pnb / 3, comp = (int)blockIdx.x / per, t = (int)blockIdx.x % per;
+    const float* const rhs = S.new_d + comp * S.pplane;
+    const float* const in = FIRST ? rhs : (parity ? S.tmp_d : S.aux_d) + comp * S.pplane;
+    float* const out = (FIRST || !parity ? S.tmp_d : S.aux_d) + comp * S.pplane;
+    if (!done)
+        poisson_flat<FIRST>(S, in, rhs, out, (unsigned)t);
 }
 
 // ---- the 12 sweeps of a small level in one launch ----
@@ -2057,9 +2097,11 @@ cudaError_t launch_cdm_poisson(const CdmSegs& L, cudaStream_t st)
     const int n = L.n - L.small;
     if (n == 0)
         return cudaSuccess;
+    const bool flat = n == 1 && (L.host[L.small].ppitch & 3);
     for (int k = 0; k < kPSweeps; ++k) {
-        auto kernel = n > 1 ? (k ? cdm_poisson_kernel<false, true> : cdm_poisson_kernel<true, true>)
-                            : (k ? cdm_poisson_kernel<false, false> : cdm_poisson_kernel<true, false>);
+        auto kernel = n > 1  ? (k ? cdm_poisson_kernel<false, true> : cdm_poisson_kernel<true, true>)
+                      : flat ? (k ? cdm_poisson_flat_kernel<false> : cdm_poisson_flat_kernel<true>)
+                             : (k ? cdm_poisson_kernel<false, false> : cdm_poisson_kernel<true, false>);
         kernel<<<L.pblocks, kPThreads, 0, st>>>(L.dev + L.small, n, L.host[L.small], k & 1);
     }
     count_launch(kPSweeps);
