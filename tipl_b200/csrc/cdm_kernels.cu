@@ -712,10 +712,15 @@ __device__ __forceinline__ double gradient_r_f32_each(const CdmSeg& S, int blk, 
                 const long long zi = i + (a <= zu ? a : zu - a) * wh;
                 for (int b = 0; b <= yu + yl; ++b) {
                     const long long yi = zi + (b <= yu ? b : yu - b) * w;
-                    for (int c = 0; c <= xu; ++c)
-                        add(yi + c);
-                    for (int c = 1; c <= xl; ++c)
-                        add(yi - c);
+                    if (w < 4)  // one loop (3x300x300 59 / 45 us), two from there on (4x300x300 89 / 73)
+                        for (int c = 0; c <= xu + xl; ++c)
+                            add(yi + (c <= xu ? c : xu - c));
+                    else {
+                        for (int c = 0; c <= xu; ++c)
+                            add(yi + c);
+                        for (int c = 1; c <= xl; ++c)
+                            add(yi - c);
+                    }
                 }
             }
             Reg r;
