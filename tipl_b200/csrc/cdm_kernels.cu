@@ -328,6 +328,8 @@ __global__ void __launch_bounds__(kCdmThreads) cdm_gradient_d_kernel(SEG_ARGS, i
 // products, along y it adds a run of 8 rows in registers, and the plane sums of the five
 // quantities go to shared memory as one uint4 a voxel (sum Js and sum It share a word: 125
 // pixels of 255 fit 16 bits); along z each thread slides the window over its (x, y) column.
+// Bound by latency at two blocks an SM (128 registers, 60 KB): at 128^3 issue 41 %, FP64 pipe and
+// conversion unit 21 and 18 %, and a warp waits 2.5 cycles an issue for its own last result.
 // Launches, per-tap byte loads and sums of 32-bit words before, so after: 157x189x155 236 / 99
 // us, 91x109x91 58.7 / 33.5, 46x55x46 17.8 / 14.7, 23x28x23 15.8 / 9.8.
 constexpr int kUX = 32, kUY = 8, kUThreads = 256;
@@ -542,8 +544,9 @@ __device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_
 // is the taps' widening to double and their products, so a thread takes V voxels in x:
 // with V = 4 a window row is 8 values, widened once (24 conversions) for 20 taps.  A square
 // of a widened float is exact, so adding it by a fused multiply-add rounds like the sum.
-// Bound by the conversion unit and the FP64 pipe (50 SM cycles each a window row of a warp of
-// 128 voxels); three blocks an SM and the tile's loads all in flight at once hide the rest.
+// Bound by latency at 24 warps an SM (80 registers): at 128^3 with every voxel inside the counters
+// read FP64 pipe 61 %, conversion unit 55 %, issue 60 %, and a warp waits 2.0 cycles an issue for
+// its own last result and 1.4 for the FP64 pipe.  The tile's loads are all in flight at once.
 // 157x189x155 launch: 305 us with one voxel a thread reading global memory, 235 so;
 // 91x109x91: 87 / 66; 64^3: 50 / 32; 23x28x23: 25 / 14.6.
 constexpr int kFX = 32, kFY = 8, kFThreads = 256, kFHX = kFX + 4, kFHY = kFY + 4, kFMaxV = 4;
